@@ -315,9 +315,9 @@ int lpm_set_kernel_timing(lpm_handle* h, int on);
  *                           folded over another number of blocks, so the
  *                           last bits differ from the graph's.
  *   LPM_CG_LOOP_AUTO        (default) persistent when the rows fit one
- *                           resident wave with a thread each and, for the
- *                           mixed solve, the FP32 operator fits in half of
- *                           L2; else the graph.
+ *                           resident wave with a thread each (and, for a
+ *                           mixed solve that cannot run on chip, the FP32
+ *                           operator fits in half of L2); else the graph.
  * Both precisions have both loops.  The matrix-free operator and kernel
  * timing always use the graph or host loop.  A barrier wait that gives up (a
  * bounded spin) ends the solve with LPM_ERR_STATE. */

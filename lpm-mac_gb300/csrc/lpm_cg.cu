@@ -1659,13 +1659,22 @@ int solve_mixed(lpm_handle* h, double tol, long long maxit, long long* iters, do
       if (st) return st;
     }
   }
-  int pthreads = 0;
-  const int pgrid = timing && !coarse ? 0 : pcg_grid(h, sv, &pthreads, coarse);
+  // the whole iteration loop on chip where one wave of blocks holds the rows
+  int pgrid = 0, pthreads = 0;
+  bool on_chip = false;
+  if (!timing && !coarse && !h->mf && h->cg_loop != LPM_CG_LOOP_GRAPH) {
+    st = pcg_run_mixed(h, (long long)h->nslots * dim * dim * 4 <= kKeepBytes);
+    if (st < 0) return st;
+    on_chip = st == 1;
+  }
+  if (!on_chip && (!timing || coarse)) pgrid = pcg_grid(h, sv, &pthreads, coarse);
   if (coarse && pgrid <= 0) {
     h->err = "coarse preconditioner: the persistent solve cannot be launched on this device";
     return LPM_ERR_STATE;
   }
-  if (pgrid > 0) {
+  if (on_chip) {
+    pgrid = 1;  // (a persistent solve, for the counters below)
+  } else if (pgrid > 0) {
     // the whole iteration loop as one persistent kernel
     st = run_persistent_mixed(h, sv, pgrid, pthreads, coarse);
     if (st) return st;

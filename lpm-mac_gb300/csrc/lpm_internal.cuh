@@ -192,6 +192,28 @@ struct Dev {
   // HCF law: per direction the tangents of the particle damage, of the
   // local and of the nonlocal damage rate [n each]
   double *tg_dD, *tg_ddot, *tg_dnl;
+  // on-chip CG solves (lpm_pcg.cu): per block the columns its rows need,
+  // their count and the position of its first row among them, per slot the
+  // column's position; (z, p) of every row, twice; the barriers' words
+  int *pl_ucnt, *pl_uown, *pl_ulist;
+  unsigned short* pl_lidx;
+  float* pl_zp;
+  unsigned long long* pl_words;
+};
+
+// Launch shape of one of the on-chip CG solves (lpm_pcg.cu).
+struct PcgShape {
+  int state = 0;  // 0 not made, 1 usable, -1 not
+  int T = 1, gs = 0, gx = 0, threads = 0;  // shares of a slice; groups kept on chip: gs per slice, one more of the first gx
+  int off_p = 0, off_list = 0, off_part = 0, off_row = 0, off_op = 0;  // shared-memory offsets
+  size_t bytes = 0;
+};
+
+// Launch plan of the on-chip CG solves, made once per handle (lpm_pcg.cu).
+struct PcgPlan {
+  int state = 0;  // 0 not made, 1 usable, -1 not
+  PcgShape mixed;
+  int G = 0, S = 0, umax = 0, smem = 0;  // blocks, slices of the largest, most columns of one, shared memory of an SM
 };
 
 // One device-resident copy of a step's state (lpm_checkpoint_save).
@@ -206,6 +228,7 @@ struct lpm_handle {
   int dim = 3, n = 0;
   int64_t nb = 0, nblk = 0;
   int64_t nslots = 0;  // sliced slots (nblk plus padding)
+  std::vector<int64_t> sell_host;  // sell_ptr on the host
   int nslice = 0;
   double particle_volume = 0;
   int nneighbors = 1;
@@ -243,6 +266,7 @@ struct lpm_handle {
   size_t ev_used = 0;
   std::vector<void*> allocations;
   std::vector<lpm::Checkpoint> checkpoints;
+  lpm::PcgPlan pcg;
   int64_t jslots = 0;  // adjoint: slots of the sliced bond data
   int tg_ndir = 0;      // tangent directions carried by the load steps (0: off)
   int tg_cap = 0;       // directions the tangent buffers hold
@@ -309,6 +333,10 @@ int solve_fp64(lpm_handle* h, double tol, long long maxit, long long* iters, dou
 int solve_mixed(lpm_handle* h, double tol, long long maxit, long long* iters, double* relres);
 int prepare_invd(lpm_handle* h, bool want32);
 int apply_operator(lpm_handle* h, int precision, const double* v_host, double* y_host);
+// the solve's loop on chip (lpm_pcg.cu), its vectors initialised and its
+// scalars in d.cg: 1 launched, 0 not possible for this system, or an error
+int pcg_plan(lpm_handle* h);
+int pcg_run_mixed(lpm_handle* h, bool keep);
 // adjoint and checkpoints (lpm_adjoint.cu); vectors are device pointers
 int adjoint_buffers(lpm_handle* h);
 int adjoint_apply(lpm_handle* h, const double* v, double* y);

@@ -393,6 +393,7 @@ int build_pattern(lpm_handle* h) {
     sp[(size_t)sl + 1] = sp[(size_t)sl] + mx * kSlice;
   }
   h->nslots = sp[(size_t)h->nslice];
+  h->sell_host = sp;
   if (h->nslots >= (int64_t)1 << 31) {
     cudaFreeAsync(cand, h->stream);
     h->err = "sliced operator has 2^31 or more slots";
