@@ -12,12 +12,12 @@
 // (boxes of an edge `box`, numbered in the order of their first particle),
 // their members, each particle's offset from its aggregate's centroid, and
 // the aggregate pairs the operator's pattern couples.  Once per assembly
-// (device): A_c in FP64, one warp per aggregate pair summing over the pair's
-// blocks in a fixed order; modes without stiffness (an aggregate whose DOFs
-// are all eliminated, the rotation of a lone particle) set aside; then the
-// inverse by Gauss-Jordan elimination without pivoting (A_c is symmetric
-// positive definite on the remaining modes), one cooperative launch with a
-// grid barrier per column.  The solve applies it in k_mx_persistent.
+// (device): A_c in FP64, one block per aggregate pair summing over the pair's
+// rows in a fixed order; then, in one cooperative launch, modes without
+// stiffness (an aggregate whose DOFs are all eliminated, the rotation of a
+// lone particle) set aside and the inverse by blocked Gauss-Jordan elimination
+// without pivoting (A_c is symmetric positive definite on the remaining modes).  The solve applies it in its own loop (lpm_pcg.cu,
+// k_mx_persistent).
 #include <algorithm>
 #include <cmath>
 #include <unordered_map>
@@ -29,80 +29,99 @@
 
 namespace lpm {
 
-// Most coarse DOFs: the dense inverse (8 MB in FP64 at 1,024) stays in L2,
-// and its Gauss-Jordan elimination takes one grid barrier per column.
+// Most coarse DOFs: the dense inverse (8 MB in FP64 at 1,024) stays in L2.
 constexpr int kCoarseMax = 1024;
 // Coarse DOFs aimed at when the box edge is chosen automatically.
 constexpr int kCoarseTarget = 480;
 
 namespace {
 
-// A_c block (a, b) = sum over i in a, blocks (i, j) with j in b, of
-// P_i^T A_ij P_j.  One warp per pair: the lanes take the pair's rows (the
-// members of a with a block in b) in turn and walk each row's slots in
-// order; the lane sums are then folded by a fixed shuffle tree.
+// out[m] += v times mode m's entry in direction k for a particle at offset
+// (dx, dy, dz): the three (2-D: two) entries that are not zero (mode_row).
 template <int DIM>
-__global__ void __launch_bounds__(128) k_coarse_pairs(int npair, const int* __restrict__ pairs,
-                                                      const int* __restrict__ prow_ptr, const int* __restrict__ prow,
-                                                      const int* __restrict__ agg, const float* __restrict__ off,
-                                                      const unsigned char* __restrict__ fixed,
-                                                      const int64_t* __restrict__ sell_ptr,
-                                                      const int* __restrict__ scol, const int* __restrict__ rowlen,
-                                                      const double* __restrict__ A, int64_t nslots, int nc,
-                                                      double* __restrict__ Ac) {
+__device__ __forceinline__ void add_modes(int k, double dx, double dy, double dz, double v,
+                                          double (&out)[kModes<DIM>]) {
+  out[k] += v;
+  if (DIM == 2) {
+    out[2] = fma(v, k == 0 ? -dy : dx, out[2]);
+  } else if (k == 0) {
+    out[4] = fma(v, dz, out[4]);
+    out[5] = fma(v, -dy, out[5]);
+  } else if (k == 1) {
+    out[3] = fma(v, -dz, out[3]);
+    out[5] = fma(v, dx, out[5]);
+  } else {
+    out[3] = fma(v, dy, out[3]);
+    out[4] = fma(v, -dx, out[4]);
+  }
+}
+
+// A_c block (a, b) = sum over i in a, blocks (i, j) with j in b, of
+// P_i^T A_ij P_j.  A block per pair: the threads take the pair's rows (the
+// members of a with a block in b) in turn, walk each row's slots in order
+// and, row by row, form A_ij P_j summed over the row before P_i^T is applied;
+// the threads' sums are folded by a fixed tree.  Bound by the FP64 pipe and
+// by the walk past the slots of other aggregates; with P_i^T applied slot by
+// slot, all modes' products taken and a warp per pair it was 10 ms for the
+// 41^3 cube.
+constexpr int kPairThreads = 128;
+template <int DIM>
+__global__ void __launch_bounds__(kPairThreads) k_coarse_pairs(const int* __restrict__ pairs,
+                                                               const int* __restrict__ prow_ptr,
+                                                               const int* __restrict__ prow,
+                                                               const int* __restrict__ agg,
+                                                               const float* __restrict__ off,
+                                                               const unsigned char* __restrict__ fixed,
+                                                               const int64_t* __restrict__ sell_ptr,
+                                                               const int* __restrict__ scol,
+                                                               const int* __restrict__ rowlen,
+                                                               const double* __restrict__ A, int64_t nslots, int nc,
+                                                               double* __restrict__ Ac) {
   constexpr int NM = kModes<DIM>;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= npair) return;
-  const int a = pairs[2 * warp], b = pairs[2 * warp + 1];
+  const int a = pairs[2 * blockIdx.x], b = pairs[2 * blockIdx.x + 1];
   double c[NM][NM];
 #pragma unroll
   for (int m = 0; m < NM; ++m)
 #pragma unroll
     for (int q = 0; q < NM; ++q) c[m][q] = 0.0;
-  for (int t = prow_ptr[warp] + lane; t < prow_ptr[warp + 1]; t += 32) {
+  for (int t = prow_ptr[blockIdx.x] + threadIdx.x; t < prow_ptr[blockIdx.x + 1]; t += kPairThreads) {
     const int i = prow[t];
-    double wi[DIM][NM];
+    double ap[DIM][NM];  // (A P)_ib
 #pragma unroll
-    for (int r = 0; r < DIM; ++r) {
-      mode_row<DIM, double>(r, off[3 * i], off[3 * i + 1], off[3 * i + 2], wi[r]);
-      if (fixed && fixed[(int64_t)DIM * i + r])
+    for (int r = 0; r < DIM; ++r)
 #pragma unroll
-        for (int m = 0; m < NM; ++m) wi[r][m] = 0.0;
-    }
+      for (int q = 0; q < NM; ++q) ap[r][q] = 0.0;
     const int len = rowlen[i];
     const SellRow sr = sell_row(sell_ptr, i);
+#pragma unroll 4
     for (int k = 0; k < len; ++k) {
-      const int64_t s = k < sr.g4 ? sr.base + (int64_t)(k / kVec) * (kSlice * kVec) + (k % kVec)
-                                  : sr.tail + (int64_t)(k - sr.g4) * kSlice;
-      const int j = scol[s];
-      if (agg[j] != b) continue;
-      double wj[DIM][NM];
+      const int64_t s = sell_slot(sr, k);
+      const int j = __ldg(&scol[s]);
+      if (__ldg(&agg[j]) != b) continue;
+      const double dx = off[3 * j], dy = off[3 * j + 1], dz = off[3 * j + 2];
 #pragma unroll
-      for (int r = 0; r < DIM; ++r) {
-        mode_row<DIM, double>(r, off[3 * j], off[3 * j + 1], off[3 * j + 2], wj[r]);
-        if (fixed && fixed[(int64_t)DIM * j + r])
+      for (int q = 0; q < DIM; ++q) {
+        if (fixed && fixed[(int64_t)DIM * j + q]) continue;
 #pragma unroll
-          for (int m = 0; m < NM; ++m) wj[r][m] = 0.0;
-      }
-      // (A_ij P_j)[r][q], then P_i^T times it
-#pragma unroll
-      for (int r = 0; r < DIM; ++r) {
-        double ap[NM];
-#pragma unroll
-        for (int q = 0; q < NM; ++q) ap[q] = 0.0;
-#pragma unroll
-        for (int s2 = 0; s2 < DIM; ++s2) {
-          const double v = A[(int64_t)(r * DIM + s2) * nslots + s];
-#pragma unroll
-          for (int q = 0; q < NM; ++q) ap[q] += v * wj[s2][q];
-        }
-#pragma unroll
-        for (int m = 0; m < NM; ++m)
-#pragma unroll
-          for (int q = 0; q < NM; ++q) c[m][q] += wi[r][m] * ap[q];
+        for (int r = 0; r < DIM; ++r)
+          add_modes<DIM>(q, dx, dy, dz, A[(int64_t)(r * DIM + q) * nslots + s], ap[r]);
       }
     }
+    const double dx = off[3 * i], dy = off[3 * i + 1], dz = off[3 * i + 2];
+#pragma unroll
+    for (int q = 0; q < NM; ++q) {
+      double col[NM];
+#pragma unroll
+      for (int m = 0; m < NM; ++m) col[m] = c[m][q];
+#pragma unroll
+      for (int r = 0; r < DIM; ++r)
+        if (!(fixed && fixed[(int64_t)DIM * i + r])) add_modes<DIM>(r, dx, dy, dz, ap[r][q], col);
+#pragma unroll
+      for (int m = 0; m < NM; ++m) c[m][q] = col[m];
+    }
   }
+  __shared__ double part[kPairThreads / 32][NM * NM];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int m = 0; m < NM; ++m)
 #pragma unroll
@@ -110,66 +129,153 @@ __global__ void __launch_bounds__(128) k_coarse_pairs(int npair, const int* __re
       double v = c[m][q];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) Ac[(int64_t)(a * NM + m) * nc + b * NM + q] = v;
+      if (lane == 0) part[warp][m * NM + q] = v;
     }
-}
-
-// Modes without stiffness: a diagonal entry at most 1e-12 of the largest.
-// Their rows and columns become those of the identity for the elimination
-// (the inverse's are cleared afterwards); `active` records which are kept.
-__global__ void k_coarse_guard(int nc, double* __restrict__ Ac, int* __restrict__ active) {
-  __shared__ double smax[32];
-  double m = 0.0;
-  for (int q = threadIdx.x; q < nc; q += blockDim.x) m = fmax(m, fabs(Ac[(int64_t)q * nc + q]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = m;
   __syncthreads();
-  m = 0.0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, smax[w]);
-  for (int q = threadIdx.x; q < nc; q += blockDim.x) active[q] = fabs(Ac[(int64_t)q * nc + q]) > 1e-12 * m ? 1 : 0;
-  __syncthreads();
-  for (int64_t e = threadIdx.x; e < (int64_t)nc * nc; e += blockDim.x) {
-    const int r = (int)(e / nc), c = (int)(e % nc);
-    if (!active[r] || !active[c]) Ac[e] = r == c ? 1.0 : 0.0;
+  for (int e = threadIdx.x; e < NM * NM; e += kPairThreads) {
+    double v = part[0][e];
+    for (int w = 1; w < kPairThreads / 32; ++w) v += part[w][e];
+    Ac[(int64_t)(a * NM + e / NM) * nc + b * NM + e % NM] = v;
   }
 }
 
-// In-place Gauss-Jordan inversion without pivoting, ping-ponged between two
-// buffers (step k reads one and writes the other), one grid barrier per
-// step.  The result is then symmetrized, (B + B^T)/2, with the rows and
-// columns of inactive modes cleared, into the other buffer (X when nc is
-// odd, else Y): elimination leaves the computed inverse of an
-// ill-conditioned A_c slightly unsymmetric, and CG needs a symmetric
-// preconditioner.
-__global__ void k_coarse_invert(int nc, double* X, double* Y, const int* __restrict__ active,
-                                unsigned long long* gbar, long long spin_limit, int* fault) {
+// The inverse of A_c by Gauss-Jordan elimination without pivoting, kInv
+// columns at a time, ping-ponged between two buffers (step k reads one and
+// writes the other).  With D the diagonal block of step k, P = D^-1 A_kj:
+//   A_kj <- P,  A_ik <- -A_ik D^-1,  A_ij <- A_ij - A_ik P,  A_kk <- D^-1.
+// A column at a time this was a grid barrier and a pass over the matrix per
+// column, 3.8 ms at 480 coarse DOFs of which the barriers were most; in
+// blocks it is two barriers and a rank-16 update per 16 columns, bound by
+// the FP64 pipe (2 nc^3 operations).  The last block of the grid takes no
+// part in the update: it works out the next step's D and inverts it
+// meanwhile, a serial chain of 16 divisions.  The whole set-up of a 61x121
+// plate (480 coarse DOFs) went from 3.9 to 0.77 ms, of a 41^3 cube from 18 to
+// 3.3 ms.
+//
+// First, modes without stiffness (a diagonal entry at most 1e-12 of the
+// largest) are set aside: their rows and columns become the identity's for
+// the elimination, and the inverse's are cleared; `active` records which
+// are kept.  The result is symmetrized, (B + B^T)/2, into the other buffer
+// (X after an odd number of steps, else Y): elimination leaves the computed
+// inverse of an ill-conditioned A_c slightly unsymmetric, and CG needs a
+// symmetric preconditioner.
+constexpr int kInv = 16;         // columns per step
+constexpr int kInvRows = 16, kInvCols = 32;  // tile of the update
+constexpr int kInvThreads = 256;
+
+// D^-1 of the block of step k after the update of step k - 1 (k > 0) applied
+// to it, into dinv (global, kInv x kInv, identity beyond the matrix).
+__device__ void invert_diagonal(int nc, int k, const double* src, const double* panel, double* dinv,
+                                double (&d)[kInv][kInv + 1]) {
+  const int r = threadIdx.x / kInv, c = threadIdx.x % kInv, i = k * kInv + r, j = k * kInv + c;
+  const bool in = i < nc && j < nc;
+  __shared__ double rp;
+  double v = in ? __ldcg(&src[(int64_t)i * nc + j]) : (r == c ? 1.0 : 0.0);
+  if (panel && in) {  // A_ij - A_i(k-1) P
+    const int k0 = (k - 1) * kInv;
+    for (int t = 0; t < kInv; ++t)
+      v -= __ldcg(&src[(int64_t)i * nc + k0 + t]) * __ldcg(&panel[(int64_t)(k0 + t) * nc + j]);
+  }
+  d[r][c] = v;
+  __syncthreads();
+  for (int p = 0; p < kInv; ++p) {
+    if (threadIdx.x == 0) rp = 1.0 / d[p][p];
+    __syncthreads();
+    const double q = rp, a = d[r][c], f = d[r][p], g = d[p][c];
+    __syncthreads();
+    if (r == p)
+      d[r][c] = c == p ? q : a * q;
+    else
+      d[r][c] = c == p ? -a * q : a - f * q * g;
+    __syncthreads();
+  }
+  dinv[threadIdx.x] = d[r][c];
+}
+
+__global__ void __launch_bounds__(kInvThreads) k_coarse_invert(int nc, double* X, double* Y, double* dinv,
+                                                               int* __restrict__ active, unsigned long long* gbar,
+                                                               long long spin_limit, int* fault) {
+  __shared__ double D[kInv][kInv + 1], L[kInvRows][kInv + 1], P[kInv][kInvCols];
+  __shared__ double smax[kInvThreads / 32];
   const int64_t nn = (int64_t)nc * nc;
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  const int last = gridDim.x - 1;  // the block that inverts; with one block it does everything
   unsigned long long target = 0;
-  for (int k = 0; k < nc; ++k) {
+  auto barrier = [&]() {
+    target += gridDim.x;
+    if (grid_barrier(gbar, target, spin_limit)) return true;
+    if (threadIdx.x == 0) atomicExch(fault, 1);
+    return false;
+  };
+  // modes without stiffness
+  {
+    double m = 0.0;
+    for (int q = threadIdx.x; q < nc; q += blockDim.x) m = fmax(m, fabs(__ldcg(&X[(int64_t)q * nc + q])));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = m;
+    __syncthreads();
+    m = 0.0;
+    for (int w = 0; w < kInvThreads / 32; ++w) m = fmax(m, smax[w]);
+    for (int64_t q = t0; q < nc; q += stride) active[q] = fabs(__ldcg(&X[q * nc + q])) > 1e-12 * m ? 1 : 0;
+    if (!barrier()) return;
+    for (int64_t e = t0; e < nn; e += stride) {
+      const int r = (int)(e / nc), c = (int)(e % nc);
+      if (!__ldcg(&active[r]) || !__ldcg(&active[c])) X[e] = r == c ? 1.0 : 0.0;
+    }
+    if (!barrier()) return;
+  }
+  if (blockIdx.x == last) invert_diagonal(nc, 0, X, nullptr, dinv, D);
+  if (!barrier()) return;
+  const int steps = (nc + kInv - 1) / kInv;
+  const int rows = (nc + kInvRows - 1) / kInvRows, cols = (nc + kInvCols - 1) / kInvCols;
+  const int workers = last > 0 ? last : 1;
+  for (int k = 0; k < steps; ++k) {
     const double* src = (k & 1) ? Y : X;
     double* dst = (k & 1) ? X : Y;
-    const double rp = 1.0 / __ldcg(&src[(int64_t)k * nc + k]);
-    for (int64_t e = t0; e < nn; e += stride) {
-      const int i = (int)(e / nc), j = (int)(e % nc);
-      double v;
-      if (i == k)
-        v = j == k ? rp : __ldcg(&src[e]) * rp;
-      else if (j == k)
-        v = -__ldcg(&src[e]) * rp;
-      else
-        v = __ldcg(&src[e]) - __ldcg(&src[(int64_t)i * nc + k]) * rp * __ldcg(&src[(int64_t)k * nc + j]);
-      dst[e] = v;
+    const double* dk = dinv + (k & 1) * kInv * kInv;
+    const int k0 = k * kInv, kb = min(kInv, nc - k0);
+    // the row panel P, and D^-1 in its place
+    for (int64_t e = t0; e < (int64_t)kb * nc; e += stride) {
+      const int r = (int)(e / nc), j = (int)(e % nc);
+      double v = 0.0;
+      if (j >= k0 && j < k0 + kb) {
+        v = __ldcg(&dk[r * kInv + j - k0]);
+      } else {
+        for (int t = 0; t < kb; ++t) v += __ldcg(&dk[r * kInv + t]) * __ldcg(&src[(int64_t)(k0 + t) * nc + j]);
+      }
+      dst[(int64_t)(k0 + r) * nc + j] = v;
     }
-    target += gridDim.x;
-    if (!grid_barrier(gbar, target, spin_limit)) {
-      if (threadIdx.x == 0) atomicExch(fault, 1);
-      return;
-    }
+    if (!barrier()) return;
+    if ((int)blockIdx.x == last && k + 1 < steps)
+      invert_diagonal(nc, k + 1, src, dst, dinv + ((k + 1) & 1) * kInv * kInv, D);
+    if ((int)blockIdx.x < workers)
+      for (int tile = blockIdx.x; tile < rows * cols; tile += workers) {
+        const int i0 = tile / cols * kInvRows, j0 = tile % cols * kInvCols;
+        __syncthreads();
+        for (int e = threadIdx.x; e < kInvRows * kInv; e += kInvThreads) {
+          const int r = e / kInv, t = e % kInv;
+          L[r][t] = i0 + r < nc && t < kb ? __ldcg(&src[(int64_t)(i0 + r) * nc + k0 + t]) : 0.0;
+        }
+        // the k-th columns take D^-1 (in dst's row panel) and start from zero
+        for (int e = threadIdx.x; e < kInv * kInvCols; e += kInvThreads) {
+          const int t = e / kInvCols, j = j0 + e % kInvCols;
+          P[t][e % kInvCols] = t < kb && j < nc ? __ldcg(&dst[(int64_t)(k0 + t) * nc + j]) : 0.0;
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < kInvRows * kInvCols; e += kInvThreads) {
+          const int r = e / kInvCols, c = e % kInvCols, i = i0 + r, j = j0 + c;
+          if (i >= nc || j >= nc || (i >= k0 && i < k0 + kb)) continue;
+          double v = j >= k0 && j < k0 + kb ? 0.0 : __ldcg(&src[(int64_t)i * nc + j]);
+#pragma unroll
+          for (int t = 0; t < kInv; ++t) v -= L[r][t] * P[t][c];
+          dst[(int64_t)i * nc + j] = v;
+        }
+      }
+    if (!barrier()) return;
   }
-  const double* res = (nc & 1) ? Y : X;
-  double* out = (nc & 1) ? X : Y;
+  const double* res = (steps & 1) ? Y : X;
+  double* out = (steps & 1) ? X : Y;
   for (int64_t e = t0; e < nn; e += stride) {
     const int i = (int)(e / nc), j = (int)(e % nc);
     out[e] = (!active[i] || !active[j]) ? 0.0 : 0.5 * (__ldcg(&res[e]) + __ldcg(&res[(int64_t)j * nc + i]));
@@ -362,8 +468,9 @@ int coarse_setup(lpm_handle* h) {
   d.cec = (double*)dev_alloc(h, sizeof(double) * nc);
   d.cz = (float*)dev_alloc(h, sizeof(float) * ndof);
   d.cfault = (int*)dev_alloc(h, sizeof(int));
+  d.cdinv = (double*)dev_alloc(h, sizeof(double) * 2 * kInv * kInv);
   if (!d.cagg || !d.cmem_ptr || !d.cmem || !d.cpair || !d.cprow_ptr || !d.cprow || !d.coff || !d.cA || !d.cA2 ||
-      !d.cact || !d.cyc || !d.cec || !d.cz || !d.cfault)
+      !d.cact || !d.cyc || !d.cec || !d.cz || !d.cfault || !d.cdinv)
     return LPM_ERR_NOMEM;
   LPM_CUDA(h, cudaMemcpyAsync(d.cagg, agg.data(), sizeof(int) * n, cudaMemcpyHostToDevice, h->stream));
   LPM_CUDA(h, cudaMemcpyAsync(d.cmem_ptr, mem_ptr.data(), sizeof(int) * (nagg + 1), cudaMemcpyHostToDevice,
@@ -396,34 +503,28 @@ int coarse_assemble(lpm_handle* h) {
   const int nc = h->cnc;
   const unsigned char* fixed = h->last_bc == LPM_BC_ELIMINATE ? d.fixed : nullptr;
   LPM_CUDA(h, cudaMemsetAsync(d.cA, 0, sizeof(double) * (size_t)nc * nc, h->stream));
-  const int warps_per_block = 4;
-  const int G = (h->cnpair + warps_per_block - 1) / warps_per_block;
-  if (G > 0) {
+  if (h->cnpair > 0) {
     if (h->dim == 3)
-      k_coarse_pairs<3><<<G, 32 * warps_per_block, 0, h->stream>>>(h->cnpair, d.cpair, d.cprow_ptr, d.cprow, d.cagg,
-                                                                  d.coff, fixed, d.sell_ptr, d.scol, d.rowlen,
-                                                                  d.A64, h->nslots, nc, d.cA);
+      k_coarse_pairs<3><<<h->cnpair, kPairThreads, 0, h->stream>>>(d.cpair, d.cprow_ptr, d.cprow, d.cagg, d.coff, fixed,
+                                                                  d.sell_ptr, d.scol, d.rowlen, d.A64, h->nslots, nc,
+                                                                  d.cA);
     else
-      k_coarse_pairs<2><<<G, 32 * warps_per_block, 0, h->stream>>>(h->cnpair, d.cpair, d.cprow_ptr, d.cprow, d.cagg,
-                                                                  d.coff, fixed, d.sell_ptr, d.scol, d.rowlen,
-                                                                  d.A64, h->nslots, nc, d.cA);
+      k_coarse_pairs<2><<<h->cnpair, kPairThreads, 0, h->stream>>>(d.cpair, d.cprow_ptr, d.cprow, d.cagg, d.coff, fixed,
+                                                                  d.sell_ptr, d.scol, d.rowlen, d.A64, h->nslots, nc,
+                                                                  d.cA);
     LPM_LAUNCHED(h, "k_coarse_pairs");
   }
-  k_coarse_guard<<<1, 1024, 0, h->stream>>>(nc, d.cA, d.cact);
-  LPM_LAUNCHED(h, "k_coarse_guard");
   if (!h->sms && cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess)
     h->sms = 1;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_coarse_invert, 256, 0) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  const long long want = ((long long)nc * nc + 255) / 256;
-  const int grid = (int)std::max<long long>(1, std::min<long long>((long long)h->sms * per_sm, want));
+  // a block per SM: the barriers cost more with more
+  const int grid = std::max(1, h->sms);
   LPM_CUDA(h, cudaMemsetAsync(d.gbar, 0, sizeof(unsigned long long), h->stream));
   LPM_CUDA(h, cudaMemsetAsync(d.cfault, 0, sizeof(int), h->stream));
   long long spin = kPcgSpinLimit;
   int ncv = nc;
-  void* args[] = {&ncv, &d.cA, &d.cA2, &d.cact, &d.gbar, &spin, &d.cfault};
-  LPM_CUDA(h, cudaLaunchCooperativeKernel((const void*)k_coarse_invert, dim3(grid), dim3(256), args, 0, h->stream));
+  void* args[] = {&ncv, &d.cA, &d.cA2, &d.cdinv, &d.cact, &d.gbar, &spin, &d.cfault};
+  LPM_CUDA(h, cudaLaunchCooperativeKernel((const void*)k_coarse_invert, dim3(grid), dim3(kInvThreads), args, 0,
+                                          h->stream));
   LPM_LAUNCHED(h, "k_coarse_invert");
   int fault = 0;
   LPM_CUDA(h, cudaMemcpyAsync(&fault, d.cfault, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -432,7 +533,7 @@ int coarse_assemble(lpm_handle* h) {
     h->err = "coarse preconditioner: a grid-barrier wait gave up in the inversion";
     return LPM_ERR_STATE;
   }
-  d.cAinv = (nc & 1) ? d.cA : d.cA2;
+  d.cAinv = ((nc + kInv - 1) / kInv & 1) ? d.cA : d.cA2;
   h->coarse_valid = true;
   return LPM_OK;
 }
