@@ -1662,13 +1662,13 @@ int solve_mixed(lpm_handle* h, double tol, long long maxit, long long* iters, do
   // the whole iteration loop on chip where one wave of blocks holds the rows
   int pgrid = 0, pthreads = 0;
   bool on_chip = false;
-  if (!timing && !coarse && !h->mf && h->cg_loop != LPM_CG_LOOP_GRAPH) {
-    st = pcg_run_mixed(h, (long long)h->nslots * dim * dim * 4 <= kKeepBytes);
+  if (coarse || (!timing && !h->mf && h->cg_loop != LPM_CG_LOOP_GRAPH)) {
+    st = pcg_run_mixed(h, (long long)h->nslots * dim * dim * 4 <= kKeepBytes, coarse);
     if (st < 0) return st;
     on_chip = st == 1;
   }
   if (!on_chip && (!timing || coarse)) pgrid = pcg_grid(h, sv, &pthreads, coarse);
-  if (coarse && pgrid <= 0) {
+  if (coarse && !on_chip && pgrid <= 0) {
     h->err = "coarse preconditioner: the persistent solve cannot be launched on this device";
     return LPM_ERR_STATE;
   }

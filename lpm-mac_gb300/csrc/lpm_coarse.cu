@@ -16,8 +16,8 @@
 // rows in a fixed order; then, in one cooperative launch, modes without
 // stiffness (an aggregate whose DOFs are all eliminated, the rotation of a
 // lone particle) set aside and the inverse by blocked Gauss-Jordan elimination
-// without pivoting (A_c is symmetric positive definite on the remaining modes).  The solve applies it in its own loop (lpm_pcg.cu,
-// k_mx_persistent).
+// without pivoting (A_c is symmetric positive definite on the remaining
+// modes).  The solve applies it in its own loop (lpm_pcg.cu, k_mx_persistent).
 #include <algorithm>
 #include <cmath>
 #include <unordered_map>
@@ -490,7 +490,7 @@ int coarse_setup(lpm_handle* h) {
   h->cnpair = (int)(pairs.size() / 2);
   h->cedge = edge;
   h->coarse_valid = false;
-  return LPM_OK;
+  return pcg_coarse_plan(h, agg, nagg);
 }
 
 // A_c of the current operator and its symmetrized inverse (in d.cAinv).

@@ -198,6 +198,9 @@ struct Dev {
   int *pl_ucnt, *pl_uown, *pl_ulist;
   unsigned short* pl_lidx;
   float* pl_zp;
+  int *pc_blk_ptr, *pc_blk_pos, *pc_blk_agg, *pc_agg_ptr;  // the coarse correction's entries (pcg_coarse_plan)
+  unsigned* pc_row;
+  float* pc_rec;
   unsigned long long* pl_words;
 };
 
@@ -205,14 +208,15 @@ struct Dev {
 struct PcgShape {
   int state = 0;  // 0 not made, 1 usable, -1 not
   int T = 1, gs = 0, gx = 0, threads = 0;  // shares of a slice; groups kept on chip: gs per slice, one more of the first gx
-  int off_p = 0, off_list = 0, off_part = 0, off_row = 0, off_op = 0;  // shared-memory offsets
+  int off_p = 0, off_list = 0, off_part = 0, off_row = 0, off_coarse = 0, off_op = 0;  // shared-memory offsets
   size_t bytes = 0;
 };
 
 // Launch plan of the on-chip CG solves, made once per handle (lpm_pcg.cu).
 struct PcgPlan {
   int state = 0;  // 0 not made, 1 usable, -1 not
-  PcgShape mixed;
+  PcgShape mixed, mixed_coarse;
+  int cmaxagg = 0, centries = 0;  // coarse correction: most aggregates a block's rows touch, (block, aggregate) pairs
   int G = 0, S = 0, umax = 0, smem = 0;  // blocks, slices of the largest, most columns of one, shared memory of an SM
 };
 
@@ -336,7 +340,8 @@ int apply_operator(lpm_handle* h, int precision, const double* v_host, double* y
 // the solve's loop on chip (lpm_pcg.cu), its vectors initialised and its
 // scalars in d.cg: 1 launched, 0 not possible for this system, or an error
 int pcg_plan(lpm_handle* h);
-int pcg_run_mixed(lpm_handle* h, bool keep);
+int pcg_run_mixed(lpm_handle* h, bool keep, bool coarse);
+int pcg_coarse_plan(lpm_handle* h, const std::vector<int>& agg, int nagg);
 // adjoint and checkpoints (lpm_adjoint.cu); vectors are device pointers
 int adjoint_buffers(lpm_handle* h);
 int adjoint_apply(lpm_handle* h, const double* v, double* y);

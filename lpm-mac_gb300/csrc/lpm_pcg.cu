@@ -42,6 +42,7 @@
 #include <cmath>
 #include <vector>
 
+#include "lpm_coarse.cuh"
 #include "lpm_device.cuh"
 #include "lpm_df.cuh"
 #include "lpm_pcg.cuh"
@@ -213,13 +214,22 @@ __device__ __forceinline__ bool poll_record(const Rec* a, Rec& r, F match) {
   return false;
 }
 
-// Sum of a pair over the warp, in every lane.
-__device__ __forceinline__ void warp_df_sum(float& s, float& c) {
+// Sums of pairs over the warp, in every lane.
+template <int K>
+__device__ __forceinline__ void warp_df_sum(float (&s)[K], float (&c)[K]) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float so = __shfl_xor_sync(0xffffffffu, s, o), co = __shfl_xor_sync(0xffffffffu, c, o);
-    df_add(s, c, so, co);
-  }
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float so = __shfl_xor_sync(0xffffffffu, s[k], o), co = __shfl_xor_sync(0xffffffffu, c[k], o);
+      df_add(s[k], c[k], so, co);
+    }
+}
+__device__ __forceinline__ void warp_df_sum(float& s, float& c) {
+  float a[1] = {s}, b[1] = {c};
+  warp_df_sum<1>(a, b);
+  s = a[0];
+  c = b[0];
 }
 
 // --------------------------------------------------------- mixed precision
@@ -321,6 +331,8 @@ struct PcgShared {
   SolveState st;
   float red[2][2][kPcgMaxSlices];
   double dred[2][kPcgMaxSlices];
+  float ye[2][32];  // coarse correction: each warp's part of y.e
+  int cdof0, cdof1, cagg0, cagg1, cent0, cent1;  // the block's coarse DOFs, aggregates and entries
   unsigned zn;  // publications of z
   int ubase[kPcgMaxSlices + 1];
 };
@@ -379,7 +391,7 @@ __device__ __forceinline__ void compute_sync(int threads) { asm volatile("bar.sy
 // take(reply, false) applies it in the other blocks.
 template <int K, typename D, typename T>
 __device__ __forceinline__ void update_sum(Rec* words, unsigned epoch, bool publish, PcgShared& sh, int S, D decide,
-                                           T take) {
+                                           T take, bool coarse = false) {
   SolveState& st = sh.st;
   const int G = gridDim.x, lane = threadIdx.x & 31;
   auto tagged = [&](const Rec& r) { return r.z == epoch; };
@@ -391,7 +403,9 @@ __device__ __forceinline__ void update_sum(Rec* words, unsigned epoch, bool publ
   if (publish) __threadfence();
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const double v = fold(lane < S ? sh.dred[k][lane] : 0.0);
+    double v = fold(lane < S ? sh.dred[k][lane] : 0.0);
+    if (coarse && k == 0)
+      v += fold(lane < (int)(blockDim.x >> 5) - 1 ? (double)sh.ye[0][lane] + (double)sh.ye[1][lane] : 0.0);
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
     if (lane == 0)
       st_rec(arrivals(words, kArrUpdate + 2 * k, epoch & 1) + blockIdx.x, (unsigned)b, (unsigned)(b >> 32), epoch, 0u);
@@ -438,12 +452,181 @@ __device__ __forceinline__ void warp_to_shared(PcgShared& sh, int ls, double (&v
     for (int k = 0; k < K; ++k) sh.dred[k][ls] = v[k];
 }
 
+// ---- coarse correction  z = D^-1 r + P A_c^-1 P^T r  (lpm_coarse.cu) ----
+// Three exchanges between the blocks, in records tagged like z: each block's
+// part of y = P^T r for the aggregates its rows touch; y, each aggregate's
+// parts summed by the block that has it (every block reading every part took
+// 10k cycles, the reads in each other's way); and e = A_c^-1 y, of which each
+// block works out a few entries (its rows of A_c^-1 stay in shared memory).
+// r.z comes as r.D^-1 r + y.e, so that no third sum over the rows is needed;
+// the e a block's rows need travel while block 0 forms beta.  Bound by those
+// trips through L2, one after the other: us per iteration here against
+// k_mx_persistent, whose grid barriers they replace, 61x121 plate (363 coarse
+// DOFs) 21 (43), 201x401 plate 25 (43), 21^3 cube 25 (65), 41^3 cube 63 (87).
+struct CoarseRow {
+  float d[3];         // offset from the aggregate's centroid
+  unsigned agg_mask;  // aggregate among the block's (low 16 bits), eliminated DOFs (bits 16..)
+};
+template <int DIM>
+struct CoarseView {
+  CoarseRow* row;     // [rows]
+  float* r;           // [DIM][rows]: r's high words
+  double* y;          // [nc]
+  double* inv;        // the block's rows of A_c^-1
+  float* e;           // the block's entries' e
+  int *pos, *agg;     // the block's entries: place among all by aggregate, aggregate
+  int rows;
+};
+template <int DIM>
+__device__ __forceinline__ CoarseView<DIM> coarse_view(const PcgMixedArgs& a) {
+  CoarseView<DIM> v;
+  v.rows = a.maxS * kSlice;
+  v.row = reinterpret_cast<CoarseRow*>(dyn + a.off_coarse);
+  v.r = reinterpret_cast<float*>(v.row + v.rows);
+  v.y = reinterpret_cast<double*>(v.r + DIM * v.rows);
+  v.inv = v.y + a.nc;
+  v.e = reinterpret_cast<float*>(v.inv + (size_t)a.cmaxrows * a.nc);
+  v.pos = reinterpret_cast<int*>(v.e + a.cmaxagg * kModes<DIM>);
+  v.agg = v.pos + a.cmaxagg;
+  return v;
+}
+// The records of publication zn: parts of y by entry, y, e.
+template <int DIM>
+__device__ __forceinline__ Rec* coarse_records(const PcgMixedArgs& a, unsigned zn) {
+  return reinterpret_cast<Rec*>(a.crec) + (size_t)(zn & 1) * ((size_t)a.centries * kModes<DIM> + 2 * (size_t)a.nc);
+}
+
+// From the rows' r (in v.r, a barrier of the compute warps before) to this
+// block's e, published, and its part of y.e in sh.ye.
+template <int DIM>
+__device__ __forceinline__ void coarse_solve(const PcgMixedArgs& a, PcgShared& sh, unsigned zn, int S) {
+  constexpr int NM = kModes<DIM>;
+  const CoarseView<DIM> v = coarse_view<DIM>(a);
+  const int nth = blockDim.x - 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = nth >> 5;
+  Rec* parts = coarse_records<DIM>(a, zn);
+  Rec* yrec = parts + (size_t)a.centries * NM;
+  Rec* erec = yrec + a.nc;
+  auto tagged = [&](const Rec& r) { return r.w == zn; };
+  const int na = sh.cent1 - sh.cent0;
+  for (int k = warp; k < na; k += nw) {
+    float sm[NM], cm[NM];
+#pragma unroll
+    for (int m = 0; m < NM; ++m) sm[m] = cm[m] = 0.f;
+    for (int s = 0; s < S; ++s) {
+      const int q = s * kSlice + lane;
+      const CoarseRow cr = v.row[q];
+      if ((int)(cr.agg_mask & 0xffffu) != k) continue;
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        if (cr.agg_mask >> (16 + c) & 1u) continue;
+        float w[NM];
+        mode_row<DIM, float>(c, cr.d[0], cr.d[1], cr.d[2], w);
+        const float rc = v.r[c * v.rows + q];
+#pragma unroll
+        for (int m = 0; m < NM; ++m)
+          if (m == c || m >= DIM) dot2_acc(sm[m], cm[m], w[m], rc);
+      }
+    }
+    warp_df_sum<NM>(sm, cm);
+    float sl = sm[0], cl = cm[0];
+#pragma unroll
+    for (int m = 1; m < NM; ++m)
+      if (lane == m) {
+        sl = sm[m];
+        cl = cm[m];
+      }
+    if (lane < NM) st_rec(parts + (size_t)v.pos[k] * NM + lane, __float_as_uint(sl), __float_as_uint(cl), 0u, zn);
+  }
+  // the block's aggregates: their parts in block order, a warp per DOF and a
+  // lane per part (an aggregate of more than 32 parts in rounds)
+  for (int c = sh.cagg0 * NM + warp; c < sh.cagg1 * NM; c += nw) {
+    const int ag = c / NM, m = c % NM;
+    float sv = 0.f, cv = 0.f;
+    for (int q = a.cagg_ptr[ag] + lane; q < a.cagg_ptr[ag + 1]; q += 32) {
+      Rec r;
+      if (!poll_record(parts + (size_t)q * NM + m, r, tagged)) sh.st.fail = 1;
+      df_add(sv, cv, __uint_as_float(r.x), __uint_as_float(r.y));
+    }
+    warp_df_sum(sv, cv);
+    if (lane == 0) st_rec(yrec + c, __float_as_uint(sv), __float_as_uint(cv), 0u, zn);
+  }
+  for (int c = threadIdx.x; c < a.nc; c += nth) {
+    Rec r;
+    if (!poll_record(yrec + c, r, tagged)) sh.st.fail = 1;
+    v.y[c] = (double)__uint_as_float(r.x) + (double)__uint_as_float(r.y);
+  }
+  compute_sync(nth);
+  float ys = 0.f, yc = 0.f;
+  for (int c = sh.cdof0 + warp; c < sh.cdof1; c += nw) {
+    const double* row = v.inv + (size_t)(c - sh.cdof0) * a.nc;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    int k = lane;
+    for (; k + 96 < a.nc; k += 128) {
+      s0 = fma(row[k], v.y[k], s0);
+      s1 = fma(row[k + 32], v.y[k + 32], s1);
+      s2 = fma(row[k + 64], v.y[k + 64], s2);
+      s3 = fma(row[k + 96], v.y[k + 96], s3);
+    }
+    for (; k < a.nc; k += 32) s0 = fma(row[k], v.y[k], s0);
+    double s[1] = {(s0 + s1) + (s2 + s3)};
+    warp_sum<1>(s);
+    if (lane == 0) {
+      const float e = (float)s[0];
+      st_rec(erec + c, __float_as_uint(e), 0u, 0u, zn);
+      float ph, pl;
+      df_split(v.y[c] * (double)e, ph, pl);
+      df_add(ys, yc, ph, pl);
+    }
+  }
+  if (lane == 0) {
+    sh.ye[0][warp] = ys;
+    sh.ye[1][warp] = yc;
+  }
+}
+
+// The e of the block's aggregates, then z of this thread's row (owner).
+template <int DIM>
+__device__ __forceinline__ void coarse_z(const PcgMixedArgs& a, PcgShared& sh, unsigned zn, const Place& pl,
+                                         float (&z)[DIM]) {
+  constexpr int NM = kModes<DIM>, E = DIM * DIM;
+  const CoarseView<DIM> v = coarse_view<DIM>(a);
+  const int nth = blockDim.x - 32, lane = threadIdx.x & 31;
+  const Rec* erec = coarse_records<DIM>(a, zn) + (size_t)a.centries * NM + a.nc;
+  const int n = (sh.cent1 - sh.cent0) * NM;
+  for (int q = threadIdx.x; q < n; q += nth) {
+    Rec r;
+    if (!poll_record(erec + v.agg[q / NM] * NM + q % NM, r, [&](const Rec& x) { return x.w == zn; })) sh.st.fail = 1;
+    v.e[q] = __uint_as_float(r.x);
+  }
+  compute_sync(nth);
+  if (pl.owner) {
+    const int q = pl.ls * kSlice + lane;
+    const CoarseRow cr = v.row[q];
+    const float* rowc = reinterpret_cast<const float*>(dyn + a.off_row) + q;
+    const float* e = v.e + (cr.agg_mask & 0xffffu) * NM;
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) {
+      float zi = rowc[(E + k) * v.rows] * v.r[k * v.rows + q];
+      if (!(cr.agg_mask >> (16 + k) & 1u)) {
+        float w[NM];
+        mode_row<DIM, float>(k, cr.d[0], cr.d[1], cr.d[2], w);
+#pragma unroll
+        for (int m = 0; m < NM; ++m) zi = fmaf(w[m], e[m], zi);
+      }
+      z[k] = zi;
+    }
+    publish_z<DIM>(a, zn, pl.row, z);
+  }
+}
+
 // Reliable update, compute warps: the solution x64 + x of every row
 // published, then r64 = s b - A64 (x64 + x) and |r64|^2; unless that ends the
 // solve, x64 += x, x = 0, r = r64 as a pair, z published, and r.z and r.p
 // give beta and the direction coefficient that restores r.p = 0
-// (k_mx_replace).  The message warp's side is update_messages.
-template <int DIM>
+// (k_mx_replace).  The message warp's side is update_messages.  (All three
+// sums in one exchange measured slower: 8.5 us against 7.7 per iteration of
+// a 41x41 plate.)
+template <int DIM, bool COARSE>
 __device__ __noinline__ void reliable_update(const PcgMixedArgs& a) {
   PcgShared& sh = block_state();
   SolveState& st = sh.st;
@@ -540,17 +723,28 @@ __device__ __noinline__ void reliable_update(const PcgMixedArgs& a) {
         z[k] = a.invd[i0 + k] * rh;
         v[0] += y[k] * (double)z[k];
         v[1] += y[k] * (double)ps[own * DIM + k];
+        if (COARSE) coarse_view<DIM>(a).r[k * a.maxS * kSlice + pl.ls * kSlice + lane] = rh;
       }
-      publish_z<DIM>(a, sh.zn + 1, pl.row, z);
+      if (!COARSE) publish_z<DIM>(a, sh.zn + 1, pl.row, z);
     }
     warp_to_shared<2>(sh, pl.ls, v);
   }
+  if (COARSE) {
+    compute_sync(nth);
+    coarse_solve<DIM>(a, sh, sh.zn + 1, pl.S);
+  }
   __syncthreads();  // r.z, r.p
+  if (COARSE) {
+    float z[DIM];
+    coarse_z<DIM>(a, sh, sh.zn + 1, pl, z);
+    compute_sync(nth);
+  }
   if (threadIdx.x == 0) sh.zn += 1;
   __syncthreads();
 }
 
 // Reliable update, message warp.
+template <bool COARSE>
 __device__ __noinline__ void update_messages(Rec* words, double threshold, unsigned epoch, int S) {
   PcgShared& sh = block_state();
   SolveState& st = sh.st;
@@ -595,7 +789,8 @@ __device__ __noinline__ void update_messages(Rec* words, double threshold, unsig
         st.zc = __uint_as_float(r.w);
         st.ru = 0;
         return Rec{};
-      });
+      },
+      COARSE);
   __syncthreads();
 }
 
@@ -639,12 +834,15 @@ __device__ __forceinline__ void alpha_sum(Rec* words, PcgShared& sh, unsigned m,
 // The second sum: |r|^2 and r.z to block 0, which forms beta and decides what
 // the solve does next.  |r|^2 is not negative, so its sign bit is the
 // arrival's tag (each copy is used every other iteration: one bit tells the
-// new record from the old).
+// new record from the old).  FIRST: before the first iteration of a solve with
+// the coarse correction, the r.z of its first direction.
+template <bool COARSE, bool FIRST = false>
 __device__ __forceinline__ void beta_sum(Rec* words, PcgShared& sh, unsigned m, unsigned epoch, int S) {
   SolveState& st = sh.st;
   const int lane = threadIdx.x & 31;
   float s0 = lane < S ? sh.red[0][0][lane] : 0.f, c0 = lane < S ? sh.red[0][1][lane] : 0.f;
   float s1 = lane < S ? sh.red[1][0][lane] : 0.f, c1 = lane < S ? sh.red[1][1][lane] : 0.f;
+  if (COARSE && lane < (int)(blockDim.x >> 5) - 1) df_add(s1, c1, sh.ye[0][lane], sh.ye[1][lane]);
   warp_df_sum(s0, c0);
   warp_df_sum(s1, c1);
   Rec* set = arrivals(words, kArrBeta, m & 1);
@@ -671,11 +869,11 @@ __device__ __forceinline__ void beta_sum(Rec* words, PcgShared& sh, unsigned m, 
     float rr, rrl, rz, rzl, bh = 0.f, bl = 0.f;
     two_sum(s0, c0, rr, rrl);
     two_sum(s1, c1, rz, rzl);
-    const long long it = st.it + 1;
+    const long long it = st.it + (FIRST ? 0 : 1);
     int done = 0, ru = 0;
     if (!isfinite(rr) || !isfinite(rz)) {
       done = 3;
-    } else {
+    } else if (!FIRST) {
       ru = rr < st.th || (rr == st.th && rrl < st.tl) || rr < (float)kRuDelta2 * st.rmax2;
       if (!ru) df_div(rz, rzl, st.zh, st.zl, bh, bl);
       if (it >= st.maxit) done = 2;
@@ -712,23 +910,29 @@ __device__ __forceinline__ void beta_sum(Rec* words, PcgShared& sh, unsigned m, 
 }
 
 // The message warp's loop.
+template <bool COARSE>
 __device__ __noinline__ void messages(Rec* words, CgScalars* cg, int S) {
   PcgShared& sh = block_state();
   SolveState& st = sh.st;
   const int lane = threadIdx.x & 31;
-  unsigned epoch = 0;
+  unsigned epoch = 0, mb = 0;  // replies, second sums
+  if (COARSE) {
+    __syncthreads();
+    beta_sum<true, true>(words, sh, mb++, ++epoch, S);
+    __syncthreads();
+  }
 #pragma unroll 1
-  for (unsigned m = 0;; ++m) {
+  for (unsigned m = 0; !(COARSE && (st.fail || st.done)); ++m) {
     __syncthreads();
     alpha_sum(words, sh, m, ++epoch, S);
     __syncthreads();
     if (st.fail) break;
     __syncthreads();
-    beta_sum(words, sh, m, ++epoch, S);
+    beta_sum<COARSE>(words, sh, mb++, ++epoch, S);
     __syncthreads();
     if (st.fail || st.done) break;
     if (st.ru) {
-      update_messages(words, cg->threshold, epoch, S);
+      update_messages<COARSE>(words, cg->threshold, epoch, S);
       epoch += 3;
       if (st.fail || st.done) break;
     }
@@ -749,7 +953,7 @@ __device__ __noinline__ void messages(Rec* words, CgScalars* cg, int S) {
 // The compute warps' iterations up to the next reliable update or the end.
 // (The reliable update and the messages are out of line: they keep no
 // registers from it.)
-template <int DIM, bool KEEP>
+template <int DIM, bool KEEP, bool COARSE>
 __device__ __forceinline__ void iterate(const PcgMixedArgs& a) {
   PcgShared& sh = block_state();
   constexpr int E = DIM * DIM;
@@ -924,8 +1128,9 @@ __device__ __forceinline__ void iterate(const PcgMixedArgs& a) {
         for (int k = 0; k < DIM; ++k) {
           df_madd(rh[k], rl[k], -ah, -al, qh[k], ql[k]);
           z[k] = rowc[(E + k) * rstride] * rh[k];
+          if (COARSE) coarse_view<DIM>(a).r[k * rstride + ls * kSlice + lane] = rh[k];
         }
-        publish_z<DIM>(a, zn, pl.row, z);
+        if (!COARSE) publish_z<DIM>(a, zn, pl.row, z);
 #pragma unroll
         for (int k = 0; k < DIM; ++k) {
           dot2_acc(sb[0], cb[0], rh[k], rh[k]);
@@ -943,7 +1148,15 @@ __device__ __forceinline__ void iterate(const PcgMixedArgs& a) {
           sh.red[k][1][ls] = cb[k];
         }
     }
+    if (COARSE) {
+      compute_sync(nth);
+      coarse_solve<DIM>(a, sh, zn, S);
+    }
     __syncthreads();  // |r|^2, r.z
+    if (COARSE) {
+      float z[DIM];
+      coarse_z<DIM>(a, sh, zn, pl, z);
+    }
     // while the sums travel: x += alpha p, and the z of the block's columns
     if (owner) {
       const float ah = st.ah, al = st.al;
@@ -973,7 +1186,7 @@ __device__ __forceinline__ void iterate(const PcgMixedArgs& a) {
   if (threadIdx.x == 0) sh.zn = zn;
 }
 
-template <int DIM, bool KEEP, int BOUND>
+template <int DIM, bool KEEP, int BOUND, bool COARSE>
 __global__ void __launch_bounds__(BOUND, 1) k_pcg_mixed(const __grid_constant__ PcgMixedArgs a) {
   constexpr int E = DIM * DIM;
   PcgShared& sh = block_state();
@@ -1011,6 +1224,15 @@ __global__ void __launch_bounds__(BOUND, 1) k_pcg_mixed(const __grid_constant__ 
     st.ah = st.al = st.bh = st.bl = 0.f;
     st.zc = 1.f;
     sh.zn = 1;
+    if (COARSE) {
+      constexpr int NM = kModes<DIM>;
+      sh.cdof0 = plan_slice(blockIdx.x, gridDim.x, a.nc);
+      sh.cdof1 = plan_slice(blockIdx.x + 1, gridDim.x, a.nc);
+      sh.cagg0 = plan_slice(blockIdx.x, gridDim.x, a.nc / NM);
+      sh.cagg1 = plan_slice(blockIdx.x + 1, gridDim.x, a.nc / NM);
+      sh.cent0 = a.cblk_ptr[blockIdx.x];
+      sh.cent1 = a.cblk_ptr[blockIdx.x + 1];
+    }
   }
   for (int u = threadIdx.x; u < U; u += blockDim.x) {
     const_cast<int*>(ul)[u] = a.ulist[(int64_t)blockIdx.x * a.umax + u];
@@ -1020,7 +1242,7 @@ __global__ void __launch_bounds__(BOUND, 1) k_pcg_mixed(const __grid_constant__ 
   __syncthreads();
   if (st.done) return;  // the same in every block
   if (comm) {
-    messages(reinterpret_cast<Rec*>(a.words), a.cg, S);
+    messages<COARSE>(reinterpret_cast<Rec*>(a.words), a.cg, S);
     return;
   }
   // the resident groups, block by block: the E elements and then the
@@ -1054,13 +1276,65 @@ __global__ void __launch_bounds__(BOUND, 1) k_pcg_mixed(const __grid_constant__ 
     // z of every row, tagged with the number of its publication, in two
     // copies by that number's parity: a block can be one publication ahead of
     // a slow reader, never two (a reader's next arrival comes after its reads)
-    publish_z<DIM>(a, 1, pl.row, z);
+    if (!COARSE) publish_z<DIM>(a, 1, pl.row, z);
+  }
+  if (COARSE) {
+    // the rows' places in the aggregates, the block's rows of A_c^-1, and the
+    // coarse-corrected z of the initial residual
+    const CoarseView<DIM> v = coarse_view<DIM>(a);
+    if (mine) {
+      CoarseRow cr{{0.f, 0.f, 0.f}, 0xffffu};
+      if (owner) {
+        cr.agg_mask = a.crow[pl.row];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) cr.d[k] = a.coff[3 * (int64_t)pl.row + k];
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) {
+          if (a.cfixed && a.cfixed[(int64_t)pl.row * DIM + k]) cr.agg_mask |= 1u << (16 + k);
+          v.r[k * v.rows + ls * kSlice + lane] = a.r[(int64_t)pl.row * DIM + k];
+        }
+      }
+      v.row[ls * kSlice + lane] = cr;
+    }
+    for (int e = threadIdx.x; e < (sh.cdof1 - sh.cdof0) * a.nc; e += nth)
+      v.inv[e] = a.cAinv[(int64_t)sh.cdof0 * a.nc + e];
+    for (int e = threadIdx.x; e < sh.cent1 - sh.cent0; e += nth) {
+      v.pos[e] = a.cblk_pos[sh.cent0 + e];
+      v.agg[e] = a.cblk_agg[sh.cent0 + e];
+    }
+    float s0 = 0.f, c0 = 0.f, s1 = 0.f, c1 = 0.f;
+    if (owner)
+#pragma unroll
+      for (int k = 0; k < DIM; ++k) {
+        const int64_t i = (int64_t)pl.row * DIM + k;
+        const float rh = a.r[i], z = rowc[(E + k) * rstride] * rh;
+        dot2_acc(s0, c0, rh, rh);
+        dot2_acc(s1, c1, rh, z);
+        c1 = fmaf(a.rlo[i], z, c1);
+      }
+    if (mine) {
+      warp_df_sum(s0, c0);
+      warp_df_sum(s1, c1);
+      if (lane == 0) {
+        sh.red[0][0][ls] = s0;
+        sh.red[0][1][ls] = c0;
+        sh.red[1][0][ls] = s1;
+        sh.red[1][1][ls] = c1;
+      }
+    }
+    compute_sync(nth);
+    coarse_solve<DIM>(a, sh, 1, S);
+    __syncthreads();
+    float z[DIM];
+    coarse_z<DIM>(a, sh, 1, pl, z);
+    __syncthreads();
+    if (st.fail || st.done) return;
   }
   compute_sync(nth);
   for (;;) {
-    iterate<DIM, KEEP>(a);
+    iterate<DIM, KEEP, COARSE>(a);
     if (st.fail || st.done) break;
-    reliable_update<DIM>(a);
+    reliable_update<DIM, COARSE>(a);
     if (st.fail || st.done) break;
   }
 }
@@ -1126,9 +1400,9 @@ namespace {
 // slice as fit, gs of every slice and one more of a block's first gx.
 // `unit` is a group's bytes, `threads` the most per block, `vec` the bytes of
 // a staged entry, `part` of a row's partial sums of one share, `rowc` of a
-// row's constants.
+// row's constants, `coarse` of the coarse correction.
 bool shape_on_plan(const lpm_handle* h, const void* fn, int threads, size_t unit, size_t vec, size_t part,
-                   size_t rowc, PcgShape* sh) {
+                   size_t rowc, size_t coarse, PcgShape* sh) {
   const PcgPlan& pl = h->pcg;
   const int maxw = threads / 32 - 1;  // compute warps
   if (pl.S > maxw) return false;
@@ -1143,7 +1417,8 @@ bool shape_on_plan(const lpm_handle* h, const void* fn, int threads, size_t unit
   sh->off_list = sh->off_p + (int)align16(vec * pl.umax);
   sh->off_part = sh->off_list + (int)align16(sizeof(int) * pl.umax);
   sh->off_row = sh->off_part + (int)align16(part * (size_t)(sh->T - 1) * pl.S * 32);
-  sh->off_op = sh->off_row + (int)align16(rowc * (size_t)pl.S * 32);
+  sh->off_coarse = sh->off_row + (int)align16(rowc * (size_t)pl.S * 32);
+  sh->off_op = sh->off_coarse + (int)align16(coarse);
   const long long room = (long long)pl.smem - sh->off_op;
   if (room < 0) return false;
   size_t units = 0;
@@ -1177,21 +1452,28 @@ bool shape_on_plan(const lpm_handle* h, const void* fn, int threads, size_t unit
   return true;
 }
 
-template <int DIM>
+template <int DIM, bool COARSE>
 int run_mixed_dim(lpm_handle* h, bool keep) {
   Dev& d = h->d;
   PcgPlan& pl = h->pcg;
   using Fn = void (*)(PcgMixedArgs);
   constexpr int kBound = kPcgThreads<DIM>, kWide = kPcgWideThreads<DIM>;
   const bool wide = (pl.S + 1) * 32 > kBound;
-  const Fn fn = wide ? (keep ? k_pcg_mixed<DIM, true, kWide> : k_pcg_mixed<DIM, false, kWide>)
-                     : (keep ? k_pcg_mixed<DIM, true, kBound> : k_pcg_mixed<DIM, false, kBound>);
-  PcgShape& sh = pl.mixed;
-  if (!sh.state)
+  const Fn fn = wide ? (keep ? k_pcg_mixed<DIM, true, kWide, COARSE> : k_pcg_mixed<DIM, false, kWide, COARSE>)
+                     : (keep ? k_pcg_mixed<DIM, true, kBound, COARSE> : k_pcg_mixed<DIM, false, kBound, COARSE>);
+  PcgShape& sh = COARSE ? pl.mixed_coarse : pl.mixed;
+  const int cmaxrows = COARSE ? (h->cnc + pl.G - 1) / pl.G : 0;
+  if (!sh.state) {
+    const size_t rows = (size_t)pl.S * kSlice;
+    const size_t coarse = COARSE ? rows * (sizeof(CoarseRow) + sizeof(float) * DIM) +
+                                       sizeof(double) * (size_t)(1 + cmaxrows) * h->cnc +
+                                       (sizeof(float) * kModes<DIM> + 2 * sizeof(int)) * (size_t)pl.cmaxagg
+                                 : 0;
     sh.state = shape_on_plan(h, (const void*)fn, wide ? kWide : kBound, kPcgUnit<DIM>, sizeof(float) * DIM,
-                             sizeof(double) * DIM, sizeof(float) * (DIM * DIM + DIM), &sh)
+                             sizeof(double) * DIM, sizeof(float) * (DIM * DIM + DIM), coarse, &sh)
                    ? 1
                    : -1;
+  }
   if (sh.state < 0) return 0;
   if (!d.pl_zp) {
     d.pl_zp = (float*)dev_alloc(h, kZBytes * (size_t)h->n);
@@ -1230,8 +1512,26 @@ int run_mixed_dim(lpm_handle* h, bool keep) {
   a.off_list = sh.off_list;
   a.off_part = sh.off_part;
   a.off_row = sh.off_row;
+  a.off_coarse = sh.off_coarse;
   a.off_op = sh.off_op;
   // tags start at 1
+  if (COARSE) {
+    a.nc = h->cnc;
+    a.cmaxrows = cmaxrows;
+    a.cmaxagg = pl.cmaxagg;
+    a.centries = pl.centries;
+    a.cblk_ptr = d.pc_blk_ptr;
+    a.cblk_pos = d.pc_blk_pos;
+    a.cblk_agg = d.pc_blk_agg;
+    a.cagg_ptr = d.pc_agg_ptr;
+    a.crow = d.pc_row;
+    a.coff = d.coff;
+    a.cfixed = h->last_bc == LPM_BC_ELIMINATE ? d.fixed : nullptr;
+    a.cAinv = d.cAinv;
+    a.crec = d.pc_rec;
+    LPM_CUDA(h, cudaMemsetAsync(d.pc_rec, 0, 16 * 2 * ((size_t)pl.centries * kModes<DIM> + 2 * (size_t)h->cnc),
+                                h->stream));
+  }
   LPM_CUDA(h, cudaMemsetAsync(d.pl_words, 0, kWordBytes, h->stream));
   LPM_CUDA(h, cudaMemsetAsync(d.pl_zp, 0, kZBytes * (size_t)h->n, h->stream));
   void* args[] = {&a};
@@ -1242,10 +1542,59 @@ int run_mixed_dim(lpm_handle* h, bool keep) {
 
 }  // namespace
 
-int pcg_run_mixed(lpm_handle* h, bool keep) {
+// The aggregates each block's rows touch (coarse_setup, when the plan is
+// usable): entries (block, aggregate) in two orders, by block and by
+// aggregate, and each row's aggregate among its block's.
+int pcg_coarse_plan(lpm_handle* h, const std::vector<int>& agg, int nagg) {
+  const int st = pcg_plan(h);
+  if (st <= 0) return st < 0 ? st : LPM_OK;
+  Dev& d = h->d;
+  PcgPlan& pl = h->pcg;
+  pl.mixed_coarse = PcgShape{};
+  std::vector<int> ptr(1, 0), blk_agg, seen((size_t)nagg, -1);
+  std::vector<unsigned> row((size_t)h->n);
+  pl.cmaxagg = 0;
+  for (int b = 0; b < pl.G; ++b) {
+    const int i0 = plan_slice(b, pl.G, h->nslice) * kSlice;
+    const int i1 = std::min(h->n, plan_slice(b + 1, pl.G, h->nslice) * kSlice);
+    const int at = (int)blk_agg.size();
+    for (int i = i0; i < i1; ++i) {
+      const int ag = agg[(size_t)i];
+      if (seen[(size_t)ag] < at) {
+        seen[(size_t)ag] = (int)blk_agg.size();
+        blk_agg.push_back(ag);
+      }
+      row[(size_t)i] = (unsigned)(seen[(size_t)ag] - at);
+    }
+    ptr.push_back((int)blk_agg.size());
+    pl.cmaxagg = std::max(pl.cmaxagg, (int)blk_agg.size() - at);
+  }
+  pl.centries = (int)blk_agg.size();
+  std::vector<int> agg_ptr((size_t)nagg + 1, 0), pos(blk_agg.size());
+  for (int ag : blk_agg) agg_ptr[(size_t)ag + 1]++;
+  for (int a = 0; a < nagg; ++a) agg_ptr[(size_t)a + 1] += agg_ptr[(size_t)a];
+  std::vector<int> fill(agg_ptr.begin(), agg_ptr.end() - 1);
+  for (size_t e = 0; e < blk_agg.size(); ++e) pos[e] = fill[(size_t)blk_agg[e]]++;
+  const int nm = h->dim == 3 ? kModes<3> : kModes<2>;
+  auto up = [&](auto** dst, const auto& v) {
+    using V = std::remove_reference_t<decltype(**dst)>;
+    *dst = (V*)dev_alloc(h, sizeof(V) * std::max<size_t>(v.size(), 1));
+    return *dst && (v.empty() || cudaMemcpyAsync(*dst, v.data(), sizeof(V) * v.size(), cudaMemcpyHostToDevice,
+                                                 h->stream) == cudaSuccess);
+  };
+  d.pc_rec = (float*)dev_alloc(h, 16 * 2 * ((size_t)pl.centries * nm + 2 * (size_t)nagg * nm));
+  if (!d.pc_rec || !up(&d.pc_blk_ptr, ptr) || !up(&d.pc_blk_pos, pos) || !up(&d.pc_blk_agg, blk_agg) ||
+      !up(&d.pc_agg_ptr, agg_ptr) || !up(&d.pc_row, row))
+    return LPM_ERR_NOMEM;
+  LPM_CUDA(h, cudaStreamSynchronize(h->stream));  // the host arrays go out of scope
+  return LPM_OK;
+}
+
+int pcg_run_mixed(lpm_handle* h, bool keep, bool coarse) {
   const int st = pcg_plan(h);
   if (st <= 0) return st;
-  return h->dim == 3 ? run_mixed_dim<3>(h, keep) : run_mixed_dim<2>(h, keep);
+  if (coarse) return h->dim == 3 ? run_mixed_dim<3, true>(h, keep) : run_mixed_dim<2, true>(h, keep);
+  return h->dim == 3 ? run_mixed_dim<3, false>(h, keep) : run_mixed_dim<2, false>(h, keep);
 }
 
 }  // namespace lpm

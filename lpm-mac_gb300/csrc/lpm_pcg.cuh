@@ -36,9 +36,20 @@ struct PcgMixedArgs {
   double *x64, *xs;  // xs: the solution a reliable update multiplies
   unsigned long long* words;
   CgScalars* cg;
+  // coarse correction: coarse DOFs and the most of a block; the entries
+  // (block, aggregate) by block (cblk_*: first, place in aggregate order,
+  // aggregate) and by aggregate (cagg_ptr); per row its aggregate among its
+  // block's; the records of y and e
+  int nc, cmaxrows, cmaxagg, centries;
+  const int *cblk_ptr, *cblk_pos, *cblk_agg, *cagg_ptr;
+  const unsigned* crow;
+  const float* coff;
+  const unsigned char* cfixed;
+  const double* cAinv;
+  float* crec;
   int64_t nslots;
   int n, nslice, umax, gs, gx, maxS, T;
-  int off_p, off_list, off_part, off_row, off_op;  // byte offsets of the dynamic shared memory's parts
+  int off_p, off_list, off_part, off_row, off_coarse, off_op;  // byte offsets of the dynamic shared memory's parts
 };
 
 }  // namespace lpm
