@@ -1163,11 +1163,32 @@ int persistent_shape(lpm_handle* h, K kernel, int cap, bool auto_ok, int slots, 
   return (int)std::max<long long>(1, g);
 }
 
+// An operator of at most this many bytes stays in L2 between the iterations.
+constexpr long long kKeepBytes = 64LL << 20;  // half of GB300's L2
+
+// A persistent FP64 solve's scalars on the host: 1, or an error.
+int persistent_done(lpm_handle* h) {
+  Dev& d = h->d;
+  LPM_CUDA(h, cudaMemcpyAsync(h->h_cg, d.cg, sizeof(CgScalars), cudaMemcpyDeviceToHost, h->stream));
+  LPM_CUDA(h, cudaStreamSynchronize(h->stream));
+  h->stats.persistent_solves += 1;
+  if (h->h_cg->pfault) {
+    h->err = "persistent solve: a grid-barrier wait gave up";
+    return LPM_ERR_STATE;
+  }
+  return 1;
+}
+
 // The FP64 solve's loop as one persistent kernel, when persistent_shape
 // allows.  Returns 1 if it ran (its scalars then in h->h_cg), 0 if the graph
 // should run, or an error.
 int run_persistent_fp64(lpm_handle* h, const SellView& sv, const double* A, double* x, double* r, double* p,
                         double* q, const double* invd) {
+  if (!h->mf && h->cg_loop != LPM_CG_LOOP_GRAPH) {  // on chip where one wave of blocks holds the rows
+    const int st = pcg_run_fp64(h, A, x, r, invd, (long long)h->nslots * h->dim * h->dim * 8 <= kKeepBytes);
+    if (st < 0) return st;
+    if (st == 1) return persistent_done(h);
+  }
   using Fn = void (*)(PcgFp64);
   const Fn fn = h->dim == 3 ? k_cg_persistent<3> : k_cg_persistent<2>;
   int threads = 0;
@@ -1179,14 +1200,7 @@ int run_persistent_fp64(lpm_handle* h, const SellView& sv, const double* A, doub
   void* args[] = {&a};
   LPM_CUDA(h, cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(threads), args, 0, h->stream));
   LPM_LAUNCHED(h, "k_cg_persistent");
-  LPM_CUDA(h, cudaMemcpyAsync(h->h_cg, d.cg, sizeof(CgScalars), cudaMemcpyDeviceToHost, h->stream));
-  LPM_CUDA(h, cudaStreamSynchronize(h->stream));
-  h->stats.persistent_solves += 1;
-  if (h->h_cg->pfault) {
-    h->err = "persistent solve: a grid-barrier wait gave up";
-    return LPM_ERR_STATE;
-  }
-  return 1;
+  return persistent_done(h);
 }
 
 cudaEvent_t next_event(lpm_handle* h) {
@@ -1337,7 +1351,6 @@ struct MixedGrids {
 // The FP32 product of a mixed solve: 16-bit column offsets when they fit;
 // the operator kept in L2 when its FP32 values take at most kKeepBytes.
 using Spmv32Fn = void (*)(SellView, const float*, const float*, float*, CgScalars*, double*, unsigned int*, float*);
-constexpr long long kKeepBytes = 64LL << 20;  // half of GB300's L2
 template <int DIM>
 Spmv32Fn spmv32_fn_dim(bool o16, bool keep) {
   if (keep) return o16 ? k_cg_spmv<float, DIM, true, true> : k_cg_spmv<float, DIM, false, true>;

@@ -207,7 +207,7 @@ struct Dev {
 // Launch shape of one of the on-chip CG solves (lpm_pcg.cu).
 struct PcgShape {
   int state = 0;  // 0 not made, 1 usable, -1 not
-  int T = 1, gs = 0, gx = 0, threads = 0;  // shares of a slice; groups kept on chip: gs per slice, one more of the first gx
+  int T = 1, gs = 0, gx = 0, tails = 0, threads = 0;  // shares of a slice; groups kept on chip: gs per slice, one more of the first gx
   int off_p = 0, off_list = 0, off_part = 0, off_row = 0, off_coarse = 0, off_op = 0;  // shared-memory offsets
   size_t bytes = 0;
 };
@@ -215,7 +215,7 @@ struct PcgShape {
 // Launch plan of the on-chip CG solves, made once per handle (lpm_pcg.cu).
 struct PcgPlan {
   int state = 0;  // 0 not made, 1 usable, -1 not
-  PcgShape mixed, mixed_coarse;
+  PcgShape mixed, mixed_coarse, fp64;
   int cmaxagg = 0, centries = 0;  // coarse correction: most aggregates a block's rows touch, (block, aggregate) pairs
   int G = 0, S = 0, umax = 0, smem = 0;  // blocks, slices of the largest, most columns of one, shared memory of an SM
 };
@@ -341,6 +341,7 @@ int apply_operator(lpm_handle* h, int precision, const double* v_host, double* y
 // scalars in d.cg: 1 launched, 0 not possible for this system, or an error
 int pcg_plan(lpm_handle* h);
 int pcg_run_mixed(lpm_handle* h, bool keep, bool coarse);
+int pcg_run_fp64(lpm_handle* h, const double* A, double* x, double* r, const double* invd, bool keep);
 int pcg_coarse_plan(lpm_handle* h, const std::vector<int>& agg, int nagg);
 // adjoint and checkpoints (lpm_adjoint.cu); vectors are device pointers
 int adjoint_buffers(lpm_handle* h);

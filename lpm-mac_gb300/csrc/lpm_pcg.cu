@@ -51,9 +51,6 @@ namespace lpm {
 namespace {
 
 constexpr int kPlanThreads = 256;
-// Polls of a record before a wait gives up: about 0.15 us each.
-constexpr long long kPollLimit = 1LL << 22;
-
 // ------------------------------------------------------------------ plan
 // Columns of the block's slices as a bitmap over all particles, in shared
 // memory (n <= 2^17: 16 KB), and for each word the number of columns below it.
@@ -148,72 +145,6 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan_fill(int n, int nslice, c
   }
 }
 
-// ---------------------------------------------------------------- messages
-// Blocks talk through 16-byte records, written and read whole (the 128-bit
-// accesses of the memory model), that carry their own tag: a reader polls the
-// record itself, so no fence and no separate flag stands between the data and
-// its use.
-struct Rec {
-  unsigned x, y, z, w;
-};
-__device__ __forceinline__ void st_rec(void* a, unsigned x, unsigned y, unsigned z, unsigned w) {
-  asm volatile(
-      "{.reg .b128 v; .reg .b64 l, h; mov.b64 l, {%1, %2}; mov.b64 h, {%3, %4}; mov.b128 v, {l, h}; "
-      "st.relaxed.gpu.global.b128 [%0], v;}" ::"l"(a),
-      "r"(x), "r"(y), "r"(z), "r"(w)
-      : "memory");
-}
-__device__ __forceinline__ Rec ld_rec(const void* a) {
-  Rec r;
-  asm volatile(
-      "{.reg .b128 v; .reg .b64 l, h; ld.relaxed.gpu.global.b128 v, [%4]; mov.b128 {l, h}, v; mov.b64 {%0, %1}, l; "
-      "mov.b64 {%2, %3}, h;}"
-      : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-      : "l"(a)
-      : "memory");
-  return r;
-}
-
-// Records of the grid sums (a.words): arrivals of the two sums of an
-// iteration and of the reliable update's, each twice (by parity), then the
-// replies.
-enum : int { kArrAlpha = 0, kArrBeta = 2, kArrUpdate = 4, kReplies = 8 };  // sets of kPcgMaxBlocks records
-constexpr int kReplyCopies = 4;  // copies of a reply, read by every fourth block
-
-__device__ __forceinline__ Rec* arrivals(Rec* words, int set, unsigned parity) {
-  return words + (size_t)(set + (int)parity) * kPcgMaxBlocks;
-}
-__device__ __forceinline__ Rec* reply(Rec* words, unsigned epoch, int copy) {
-  return words + (size_t)kReplies * kPcgMaxBlocks + ((epoch & 1) * kReplyCopies + copy) * 8;  // 128 bytes apart
-}
-
-// One record per lane and stride of 32 blocks, polled until match() accepts
-// it; bounded.
-template <typename F>
-__device__ __forceinline__ bool gather_records(const Rec* set, int G, Rec (&r)[kPcgMaxBlocks / 32], F match) {
-  const int lane = threadIdx.x & 31;
-  for (long long polls = 0; polls < kPollLimit; ++polls) {
-#pragma unroll
-    for (int q = 0; q < kPcgMaxBlocks / 32; ++q)
-      if (lane + 32 * q < G) r[q] = ld_rec(set + lane + 32 * q);
-    bool all = true;
-#pragma unroll
-    for (int q = 0; q < kPcgMaxBlocks / 32; ++q)
-      if (lane + 32 * q < G) all = all && match(r[q]);
-    if (__all_sync(0xffffffffu, all)) return true;
-  }
-  return false;
-}
-
-template <typename F>
-__device__ __forceinline__ bool poll_record(const Rec* a, Rec& r, F match) {
-  for (long long polls = 0; polls < kPollLimit; ++polls) {
-    r = ld_rec(a);
-    if (match(r)) return true;
-  }
-  return false;
-}
-
 // Sums of pairs over the warp, in every lane.
 template <int K>
 __device__ __forceinline__ void warp_df_sum(float (&s)[K], float (&c)[K]) {
@@ -235,14 +166,6 @@ __device__ __forceinline__ void warp_df_sum(float& s, float& c) {
 // --------------------------------------------------------- mixed precision
 constexpr double kRuDelta2 = 0.1 * 0.1;  // reliable-update trigger on |r|^2 (kDelta of lpm_cg.cu squared)
 
-template <int DIM>
-__device__ __forceinline__ unsigned comp_u16(const ushort4& v, int t) {
-  return t == 0 ? v.x : t == 1 ? v.y : t == 2 ? v.z : v.w;
-}
-__device__ __forceinline__ float comp_f(const float4& v, int t) {
-  return t == 0 ? v.x : t == 1 ? v.y : t == 2 ? v.z : v.w;
-}
-
 // One block of a row (element e from at(e)) times the staged difference p - pi,
 // compensated.
 template <int DIM, typename F>
@@ -261,22 +184,6 @@ __device__ __forceinline__ void block_acc(F at, const float* p, const float (&pi
   for (int r = 0; r < DIM; ++r)
 #pragma unroll
     for (int k = 0; k < DIM; ++k) dot2_acc(s[r], c[r], at(r * DIM + k), pc[k]);
-}
-
-// Groups of a slice in the order the solve takes them: the tail of at most
-// three single blocks first (as a group padded with zeros, when the slice
-// has one), then the groups of four.
-struct SliceGroups {
-  int64_t base;  // first slot of the slice
-  int g4;        // blocks in groups of four
-  int tail;      // blocks after them
-  int count;     // groups, the tail included
-};
-__device__ __forceinline__ SliceGroups slice_groups(const int64_t* __restrict__ sell_ptr, int slice) {
-  const int64_t b = sell_ptr[slice];
-  const int w = (int)((sell_ptr[slice + 1] - b) / kSlice);
-  const int g4 = w / kVec * kVec;
-  return SliceGroups{b, g4, w - g4, g4 / kVec + (w > g4 ? 1 : 0)};
 }
 
 template <int DIM, bool KEEP>
@@ -354,35 +261,11 @@ __device__ __forceinline__ void df_div(float ah, float al, float bh, float bl, f
   two_sum(q1, q2, qh, ql);
 }
 
-// A compute thread's place: its slice among the block's, its share of the
-// slice's groups, its row.  A block with fewer slices than the widest leaves
-// its last warps without a share.  The block's last warp computes nothing: it
-// carries the messages, in a loop of its own.
-struct Place {
-  int s0, S, ls, t, row;
-  bool act, mine, owner;  // has a share; owns the slice's rows; owns a row
-};
-__device__ __forceinline__ Place place_of(const PcgMixedArgs& a) {
-  Place p;
-  p.s0 = plan_slice(blockIdx.x, gridDim.x, a.nslice);
-  p.S = plan_slice(blockIdx.x + 1, gridDim.x, a.nslice) - p.s0;
-  const int warp = threadIdx.x >> 5;
-  p.ls = warp % p.S;
-  p.t = warp / p.S;
-  p.row = (p.s0 + p.ls) * kSlice + (int)(threadIdx.x & 31);
-  p.act = p.t < a.T;
-  p.mine = p.t == 0;
-  p.owner = p.mine && p.row < a.n;
-  return p;
-}
 template <int DIM>
 __device__ __forceinline__ void publish_z(const PcgMixedArgs& a, unsigned zn, int row, const float (&z)[DIM]) {
   st_rec(reinterpret_cast<Rec*>(a.zp) + (size_t)(zn & 1) * a.n + row, __float_as_uint(z[0]), __float_as_uint(z[1]),
          DIM == 3 ? __float_as_uint(z[DIM - 1]) : 0u, zn);
 }
-
-// Barrier of the compute warps alone.
-__device__ __forceinline__ void compute_sync(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 
 // The message warp's part of a grid sum of the reliable update: K <= 2 FP64
 // values per block from sh.dred, the blocks' writes before it visible after
@@ -1068,7 +951,7 @@ __device__ __forceinline__ void iterate(const PcgMixedArgs& a) {
         kn += a.T;
 #pragma unroll
         for (int q = 0; q < kVec; ++q)
-          block_acc<DIM>([&](int e) { return comp_f(an[e], q); }, ps + comp_u16<DIM>(ln, q) * DIM, pi, qh, ql);
+          block_acc<DIM>([&](int e) { return comp_f(an[e], q); }, ps + comp_u16(ln, q) * DIM, pi, qh, ql);
         if (kn < sg.count) load_group<DIM, KEEP>(a, sg, kn, lane, an, ln, own);
       }
     }
@@ -1259,7 +1142,7 @@ __global__ void __launch_bounds__(BOUND, 1) k_pcg_mixed(const __grid_constant__ 
         float* b = reinterpret_cast<float*>(unit + (size_t)k * kPcgUnit<DIM> + q * kBlk);
 #pragma unroll
         for (int e = 0; e < E; ++e) b[e * 32 + lane] = comp_f(v[e], q);
-        reinterpret_cast<unsigned short*>(b + E * 32)[lane] = (unsigned short)comp_u16<DIM>(l, q);
+        reinterpret_cast<unsigned short*>(b + E * 32)[lane] = (unsigned short)comp_u16(l, q);
       }
     }
   if (owner) {
@@ -1339,12 +1222,14 @@ __global__ void __launch_bounds__(BOUND, 1) k_pcg_mixed(const __grid_constant__ 
   }
 }
 
-// Bytes of the grid sums' records, and per row of the two copies of z.
-constexpr size_t kWordBytes = 16 * ((size_t)kReplies * kPcgMaxBlocks + 2 * kReplyCopies * 8), kZBytes = 32;
-
-size_t align16(size_t b) { return (b + 15) / 16 * 16; }
-
 }  // namespace
+
+// No memory for the plan: the other loops need none of it.
+static int pcg_no_memory(lpm_handle* h) {
+  cudaGetLastError();
+  h->err.clear();
+  return 0;
+}
 
 // The column plan of the handle's pattern, once: 1 if the solves of this
 // file can run on it, 0 if not (more rows than one wave of blocks holds, or
@@ -1363,10 +1248,10 @@ int pcg_plan(lpm_handle* h) {
   if (S > kPcgMaxSlices) return 0;
   const int words = (h->n + 31) / 32;
   if ((size_t)words * 8 > 48 * 1024) return 0;
-  d.pl_ucnt = (int*)zeros_dev(h, sizeof(int) * G);
+  d.pl_ucnt = (int*)dev_alloc(h, sizeof(int) * G);
   d.pl_uown = (int*)dev_alloc(h, sizeof(int) * G);
-  if (!d.pl_ucnt || !d.pl_uown) return LPM_ERR_NOMEM;
-  LPM_CUDA(h, cudaStreamSynchronize(0));  // the zero fill, which is not ordered with the handle's stream
+  if (!d.pl_ucnt || !d.pl_uown) return pcg_no_memory(h);
+  LPM_CUDA(h, cudaMemsetAsync(d.pl_ucnt, 0, sizeof(int) * G, h->stream));
   k_plan_count<<<G, kPlanThreads, (size_t)words * 4, h->stream>>>(h->n, h->nslice, d.sell_ptr, d.scol, d.rowlen,
                                                                   d.pl_ucnt);
   LPM_LAUNCHED(h, "k_plan_count");
@@ -1378,7 +1263,8 @@ int pcg_plan(lpm_handle* h) {
   d.pl_ulist = (int*)dev_alloc(h, sizeof(int) * (size_t)G * umax);
   d.pl_lidx = (unsigned short*)dev_alloc(h, sizeof(unsigned short) * (size_t)std::max<int64_t>(h->nslots, 1));
   d.pl_words = (unsigned long long*)dev_alloc(h, kWordBytes);
-  if (!d.pl_ulist || !d.pl_lidx || !d.pl_words) return LPM_ERR_NOMEM;
+  d.pl_zp = (float*)dev_alloc(h, kZBytes64 * (size_t)h->n);
+  if (!d.pl_ulist || !d.pl_lidx || !d.pl_words || !d.pl_zp) return pcg_no_memory(h);
   // slots of the rows past the last particle stay at position 0
   LPM_CUDA(h, cudaMemsetAsync(d.pl_lidx, 0, sizeof(unsigned short) * (size_t)std::max<int64_t>(h->nslots, 1),
                               h->stream));
@@ -1394,6 +1280,8 @@ int pcg_plan(lpm_handle* h) {
 }
 
 namespace {
+
+size_t align16(size_t b) { return (b + 15) / 16 * 16; }
 
 // Launch shape of a solve on the plan, worked out once per handle: the
 // staged vector, its columns, the row data, then as many operator groups per
@@ -1443,7 +1331,8 @@ bool shape_on_plan(const lpm_handle* h, const void* fn, int threads, size_t unit
   sh->bytes = (size_t)sh->off_op + units * unit;
   sh->threads = (pl.S * sh->T + 1) * 32;
   int per_sm = 0;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh->bytes) != cudaSuccess ||
+  // (the attribute belongs to the kernel, not to the handle: always the most)
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, sh->threads, sh->bytes) != cudaSuccess ||
       per_sm < 1) {
     cudaGetLastError();
@@ -1475,10 +1364,6 @@ int run_mixed_dim(lpm_handle* h, bool keep) {
                    : -1;
   }
   if (sh.state < 0) return 0;
-  if (!d.pl_zp) {
-    d.pl_zp = (float*)dev_alloc(h, kZBytes * (size_t)h->n);
-    if (!d.pl_zp) return LPM_ERR_NOMEM;
-  }
   PcgMixedArgs a{};
   a.sell_ptr = d.sell_ptr;
   a.ucnt = d.pl_ucnt;
@@ -1584,8 +1469,10 @@ int pcg_coarse_plan(lpm_handle* h, const std::vector<int>& agg, int nagg) {
   };
   d.pc_rec = (float*)dev_alloc(h, 16 * 2 * ((size_t)pl.centries * nm + 2 * (size_t)nagg * nm));
   if (!d.pc_rec || !up(&d.pc_blk_ptr, ptr) || !up(&d.pc_blk_pos, pos) || !up(&d.pc_blk_agg, blk_agg) ||
-      !up(&d.pc_agg_ptr, agg_ptr) || !up(&d.pc_row, row))
-    return LPM_ERR_NOMEM;
+      !up(&d.pc_agg_ptr, agg_ptr) || !up(&d.pc_row, row)) {
+    pl.mixed_coarse.state = -1;
+    pcg_no_memory(h);
+  }
   LPM_CUDA(h, cudaStreamSynchronize(h->stream));  // the host arrays go out of scope
   return LPM_OK;
 }

@@ -49,7 +49,7 @@ CASES = {
 }
 
 
-def _solve(case, precision, damage=False, loop=capi.CG_LOOP_AUTO):
+def _solve(case, precision, damage=False, loop=capi.CG_LOOP_AUTO, maxit=-1):
     dim, xyz, p1, p2, layer, Kn, Tv, cell = case
     g = make_gpu(dim, xyz, p1, p2, layer, Kn, Tv, cell)
     rng = np.random.default_rng(9)
@@ -67,7 +67,7 @@ def _solve(case, precision, damage=False, loop=capi.CG_LOOP_AUTO):
     g.upload(capi.F_RESIDUAL, b.ravel())
     g.set_cg_loop(loop)
     g.reset_stats()
-    it, rr, st = g.solve(precision, TOL)
+    it, rr, st = g.solve(precision, TOL, maxit=maxit)
     x, on_chip = g.download(capi.F_DISP), g.stats()["persistent_solves"]
     A = dense_from_bsr(*g.pattern(), g.K_bsr(), g.n, dim).T
     g.close()
@@ -86,6 +86,47 @@ def test_mixed_solve_on_chip(name):
     print("[on chip] %s: %d iterations, residual %.2e of a bound of %.2e" % (name, it, r, bound))
     assert st == capi.OK and on_chip == 1
     assert r <= bound
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_fp64_solve_on_chip(name):
+    _solve(CASES["cube 12"](), capi.PREC_MIXED)  # other data left in the SMs' shared memory
+    A, b, x, it, st, on_chip = _solve(CASES[name](), capi.PREC_FP64)
+    r, bound = _held(A, b, x)
+    print("[on chip] %s: %d FP64 iterations, residual %.2e of a bound of %.2e" % (name, it, r, bound))
+    assert st == capi.OK and on_chip == 1
+    assert r <= bound
+
+
+def test_fp64_solve_stops_at_the_limit():
+    """At a limit of 7 iterations, the graph loop's iterate to rounding."""
+    case = plate(17, 23)
+    _, b, x, it, st, on_chip = _solve(case, capi.PREC_FP64, maxit=7)
+    _, _, xg, itg, stg, _ = _solve(case, capi.PREC_FP64, maxit=7, loop=capi.CG_LOOP_GRAPH)
+    assert on_chip == 1 and it == itg == 7 and st == stg == capi.NOT_CONVERGED
+    assert np.abs(x - xg).max() <= 1e-13 * np.abs(xg).max() * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("precision", [capi.PREC_MIXED, capi.PREC_FP64])
+def test_handles_of_two_sizes_in_turn(precision):
+    """A small system's solve between two of a larger one: the launch limits
+    are the kernel's, not the handle's."""
+    big, small = make_gpu(*plate(40, 60)), make_gpu(*plate(5, 5))
+    res = []
+    for g in (big, small, big):
+        mask = np.zeros((g.n, 3), np.int32)
+        mask[:9, :2] = 1
+        g.set_mask(mask)
+        g.update()
+        g.assemble(capi.TANGENT_SYMMETRIC, capi.BC_ELIMINATE)
+        b = np.random.default_rng(g.n).standard_normal((g.n, 2)) * (1 - mask[:, :2])
+        g.upload(capi.F_RESIDUAL, b.ravel())
+        g.reset_stats()
+        assert g.solve(precision, TOL)[2] == capi.OK and g.stats()["persistent_solves"] == 1
+        res.append(g.download(capi.F_DISP))
+    assert np.array_equal(res[0], res[2])
+    big.close()
+    small.close()
 
 
 def test_mixed_solve_on_chip_with_damage():
