@@ -108,6 +108,8 @@ struct Dev {
   // bonds
   int64_t *bptr, *lptr;
   int *bp2, *blayer, *opp;
+  double* brec;  // an assembly's bond records (lpm_tangent.cu)
+  int* sopp;
   int *sbond, *sp2;  // per (particle, layer) segment: bond ids and partners sorted by partner id
   double *Kn, *Tv, *dis0, *dis, *dis_last, *dLe, *dLp, *dLp_last, *bstrain, *cs, *bforce, *bforce_last, *bdamage,
       *bdamage_last;
@@ -233,6 +235,8 @@ struct lpm_handle {
   int64_t nb = 0, nblk = 0;
   int64_t nslots = 0;  // sliced slots (nblk plus padding)
   std::vector<int64_t> sell_host;  // sell_ptr on the host
+  int maxw = 0;                    // blocks of the widest slice
+  bool no_records = false;         // no memory for the bond records
   int nslice = 0;
   double particle_volume = 0;
   int nneighbors = 1;

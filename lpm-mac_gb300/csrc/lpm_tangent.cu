@@ -7,10 +7,10 @@
 //
 // Tangent (stiffness.h:67-101, 228-263; derivative.h): block K_ij for every
 // j in conns(i).  The stored operator is A = K^T (see lpm_internal.cuh); a
-// warp owns one row j of A and its lanes compute the blocks K_ij, i in
-// conns(j), each by walking the bond lists exactly as derivative.h does, so
-// the terms of a block are added in the reference's order.
+// lane owns a row j of A and computes blocks K_ij, i in conns(j), each by a
+// merge of the two particles' bond lists.
 #include <algorithm>
+#include <climits>
 #include <numeric>
 
 #include "lpm_device.cuh"
@@ -103,10 +103,14 @@ __global__ void k_fill_sell(int n, const int64_t* __restrict__ cptr, const int* 
   diag_slot[j] = ds;
 }
 
+constexpr int kAsmThreads = 512;  // most warps of a slice: 16 groups
+
 struct AsmView {
   const int64_t *bptr, *lptr, *sell_ptr;
   const int *scol, *rowlen, *sbond, *sp2, *opp;
   const double *cs, *cs_sum, *tsum, *msum, *Kn, *Tv, *bdamage;
+  const double2* rec;  // per sorted bond {n, w Tv / 2}, and the sorted place of its opposite (bond_records), or null
+  const int* sopp;
   double* A;
   int64_t nslots;
   int n, nslice, sym;
@@ -156,104 +160,139 @@ __device__ __forceinline__ void diag_block(const AsmView& v, int i, double (&K)[
   K[2][2] = k22;
 }
 
-constexpr int kMatch = 8;  // common neighbours collected per merge chunk
+// A bond's direction cosines and half its damaged Tv.
+struct BondRec {
+  double n[3], t;
+};
+__device__ __forceinline__ BondRec bond_rec(const AsmView& v, int64_t b) {
+  return BondRec{{v.cs[3 * b], v.cs[3 * b + 1], v.cs[3 * b + 2]}, 0.5 * ((1 - v.bdamage[b]) * v.Tv[b])};
+}
+// Of the bond at sorted place s, and of its opposite.
+template <bool REC>
+__device__ __forceinline__ BondRec own_rec(const AsmView& v, int64_t s) {
+  if (!REC) return bond_rec(v, v.sbond[s]);
+  const double2 a = __ldg(v.rec + 2 * s), b = __ldg(v.rec + 2 * s + 1);
+  return BondRec{{a.x, a.y, b.x}, b.y};
+}
+template <bool REC>
+__device__ __forceinline__ BondRec opp_rec(const AsmView& v, int64_t s) {
+  return REC ? own_rec<true>(v, __ldg(v.sopp + s)) : bond_rec(v, v.opp[v.sbond[s]]);
+}
 
-template <int DIM>
+__global__ void k_bond_records(int64_t nb, const int* __restrict__ sbond, const double* __restrict__ cs,
+                               const double* __restrict__ Tv, const double* __restrict__ bdamage,
+                               double2* __restrict__ rec) {
+  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < nb; s += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = sbond[s];
+    rec[2 * s] = make_double2(cs[3 * b], cs[3 * b + 1]);
+    rec[2 * s + 1] = make_double2(cs[3 * b + 2], 0.5 * ((1 - bdamage[b]) * Tv[b]));
+  }
+}
+__global__ void k_sorted_place(int64_t nb, const int* __restrict__ sbond, int* __restrict__ place) {
+  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < nb; s += (int64_t)gridDim.x * blockDim.x)
+    place[sbond[s]] = (int)s;
+}
+__global__ void k_sorted_opp(int64_t nb, const int* __restrict__ sbond, const int* __restrict__ opp,
+                             const int* __restrict__ place, int* __restrict__ sopp) {
+  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < nb; s += (int64_t)gridDim.x * blockDim.x)
+    sopp[s] = place[opp[sbond[s]]];
+}
+
+template <int DIM, bool REC>
 __device__ __forceinline__ void off_block(const AsmView& v, int i, int j, double (&K)[3][3]) {
 #pragma unroll
   for (int r = 0; r < 3; ++r)
 #pragma unroll
     for (int c = 0; c < 3; ++c) K[r][c] = 0.0;
+#pragma unroll 1
   for (int l = 0; l < NL; ++l) {
-    double B[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) B[r][c] = 0.0;
     int64_t ia, ea, ib, eb;
     seg(v.bptr, v.lptr, i, l, ia, ea);
     seg(v.bptr, v.lptr, j, l, ib, eb);
-    int direct = -1;
+    int64_t direct = -1;
+    int pb = ib < eb ? __ldg(v.sp2 + ib) : INT_MAX;
     // merge of the partner-sorted lists; the direct bond i->j shows up as
-    // partner j in i's list.  The common neighbours are collected kMatch at
-    // a time and their FP64 terms added after the (integer) merge, in merge
-    // order: the lanes of a warp then run the FP64 work together instead of
-    // each at its own point of the merge.
-    while (ia < ea) {
-      int m1[kMatch], m3[kMatch];
-      int nm = 0;
-      while (ia < ea && nm < kMatch) {
-        const int pa = v.sp2[ia];
-        if (pa == j) direct = v.sbond[ia];
-        while (ib < eb && v.sp2[ib] < pa) ++ib;
-        if (ib < eb && v.sp2[ib] == pa) {
-          m1[nm] = v.sbond[ia];          // i -> k
-          m3[nm] = v.opp[v.sbond[ib]];   // k -> j, opposite of j -> k
-          ++nm;
+    // partner j in i's list.  The lanes of a warp walk (integers) each to
+    // its next common neighbour and then take its FP64 terms together.
+#pragma unroll 1
+    for (;;) {
+      bool match = false;
+#pragma unroll 1
+      for (; ia < ea; ++ia) {
+        const int pa = __ldg(v.sp2 + ia);
+        if (pa == j) direct = ia;
+        while (pb < pa) pb = ++ib < eb ? __ldg(v.sp2 + ib) : INT_MAX;
+        if (pb == pa) {
+          match = true;
+          break;
         }
-        ++ia;
       }
-      for (int t = 0; t < nm; ++t) {
-        const int b1 = m1[t], b3 = m3[t];
-        const double h = 0.5 * ((1 - v.bdamage[b3]) * v.Tv[b3] + (1 - v.bdamage[b1]) * v.Tv[b1]);
-        const double n1[3] = {v.cs[3 * (int64_t)b1], v.cs[3 * (int64_t)b1 + 1], v.cs[3 * (int64_t)b1 + 2]};
-        const double n3[3] = {v.cs[3 * (int64_t)b3], v.cs[3 * (int64_t)b3 + 1], v.cs[3 * (int64_t)b3 + 2]};
+      if (!match) break;
+      const BondRec a = own_rec<REC>(v, ia++), b = opp_rec<REC>(v, ib);  // i -> k, k -> j
+      const double h = a.t + b.t;
 #pragma unroll
-        for (int r = 0; r < DIM; ++r) {
-          const double hr = h * n1[r];
+      for (int r = 0; r < DIM; ++r) {
+        const double hr = h * a.n[r];
 #pragma unroll
-          for (int c = 0; c < DIM; ++c) B[r][c] -= hr * n3[c];
-        }
+        for (int c = 0; c < DIM; ++c) K[r][c] = fma(-hr, b.n[c], K[r][c]);
       }
     }
     if (direct >= 0) {
-      const int64_t b = direct;
-      const double n[3] = {v.cs[3 * b], v.cs[3 * b + 1], v.cs[3 * b + 2]};
-      const double w = 1 - v.bdamage[b], kn = v.Kn[b], tv = v.Tv[b], kt = kn + tv, wt = w * tv;
+      const BondRec a = own_rec<REC>(v, direct);
+      const int64_t b = v.sbond[direct];
+      const double wt = 2.0 * a.t, wn = 2.0 * ((1 - v.bdamage[b]) * v.Kn[b]) + wt;
       const double* Sj = v.cs_sum + (NL * j + l) * 3;
       const double* Si = v.cs_sum + (NL * i + l) * 3;
       const double* Ti = v.tsum + (NL * i + l) * 3;
+      double p[DIM];
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) p[c] = fma(wt, Sj[c], -(wn * a.n[c]));
 #pragma unroll
       for (int r = 0; r < DIM; ++r) {
-        const double o = 0.5 * (wt * (Si[r] - n[r]) + (Ti[r] - wt * n[r]));
+        const double o = fma(0.5, fma(wt, Si[r], Ti[r]), -(wt * a.n[r]));
 #pragma unroll
-        for (int c = 0; c < DIM; ++c)
-          B[r][c] += w * ((-kn * n[c] + tv * Sj[c]) * n[r] - kt * n[r] * n[c]) - o * n[c];
+        for (int c = 0; c < DIM; ++c) K[r][c] = fma(a.n[r], p[c], fma(-o, a.n[c], K[r][c]));
       }
     }
-#pragma unroll
-    for (int r = 0; r < DIM; ++r)
-#pragma unroll
-      for (int c = 0; c < DIM; ++c) K[r][c] += B[r][c];
   }
 }
 
-// One warp per slice of A = K^T: lane t owns row j = 32*slice + t and,
-// column by column (k), computes block K_ij with i the k-th entry of conns(j)
-// and stores its transpose in the row's k-th slot.
-template <int DIM>
-__global__ void __launch_bounds__(256) k_assemble(AsmView v) {
-  const int lane = threadIdx.x & 31;
-  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long sl = w0; sl < v.nslice; sl += nw) {
-    const int j = (int)(sl * kSlice) + lane;
-    const int len = j < v.n ? v.rowlen[j] : 0;
-    const SellRow row = j < v.n ? sell_row(v.sell_ptr, j) : SellRow{0, 0, 0};
-    for (int k = 0; k < len; ++k) {
+// A block per slice of A = K^T: lane t owns row j = 32*slice + t, the warps
+// share the row's blocks, four (a group) at a time.  Each computes K_ij with
+// i the k-th entry of conns(j) and stores its transpose in the row's k-th
+// slot: on a lattice the lanes' k-th blocks see the same neighbourhood, so
+// they walk and multiply together.
+//
+// Bound by the FP64 pipe (13 operations per common neighbour and layer, 36 per
+// direct bond: 0.6 ms of 51^3 particles) and, next, by the L1's accesses: a
+// lane's list and records lie apart from its neighbour's.  The records bring
+// a bond's data in two loads instead of seven (sorted place, bond, its
+// opposite, four arrays).  With one warp per slice and the raw arrays it was
+// latency: 0.33 ms for any plate up to 7k rows (now 0.08 with the conditions), 1.2
+// for a 21^3 cube (0.26), 2.9 for 51^3 (1.6), 17.8 for 101^3 (8.9).
+template <int DIM, bool REC>
+__global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmView v) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int j = blockIdx.x * kSlice + lane;
+  if (j >= v.n) return;
+  const int len = v.rowlen[j];
+  const SellRow row = sell_row(v.sell_ptr, j);
+#pragma unroll 1
+  for (int g = warp * kVec; g < len; g += nw * kVec)
+#pragma unroll 1
+    for (int k = g; k < min(len, g + kVec); ++k) {
       const int64_t slot = sell_slot(row, k);
       const int i = v.scol[slot];
       double K[3][3];
       if (i == j)
         diag_block<DIM>(v, i, K);
       else
-        off_block<DIM>(v, i, j, K);
+        off_block<DIM, REC>(v, i, j, K);
 #pragma unroll
       for (int r = 0; r < DIM; ++r)
 #pragma unroll
         for (int s = 0; s < DIM; ++s) v.A[(r * DIM + s) * v.nslots + slot] = K[s][r];
     }
-  }
 }
 
 // |diag(K)|_2 (stiffness.h:269-270) and the DOFs to eliminate
@@ -394,6 +433,9 @@ int build_pattern(lpm_handle* h) {
   }
   h->nslots = sp[(size_t)h->nslice];
   h->sell_host = sp;
+  h->maxw = 0;
+  for (int sl = 0; sl < h->nslice; ++sl)
+    h->maxw = std::max(h->maxw, (int)((sp[(size_t)sl + 1] - sp[(size_t)sl]) / kSlice));
   if (h->nslots >= (int64_t)1 << 31) {
     cudaFreeAsync(cand, h->stream);
     h->err = "sliced operator has 2^31 or more slots";
@@ -422,6 +464,33 @@ int build_pattern(lpm_handle* h) {
   return LPM_OK;
 }
 
+// The bonds' records of an assembly: 1 made, 0 no memory for them, or an error.
+static int bond_records(lpm_handle* h) {
+  Dev& d = h->d;
+  if (h->no_records || h->nb == 0) return 0;
+  const int T = 256, G = grid_for((long long)h->nb, T, 152 * 32);
+  if (!d.brec) {
+    d.brec = (double*)dev_alloc(h, sizeof(double) * 4 * (size_t)h->nb);
+    if (d.brec) d.sopp = (int*)dev_alloc(h, sizeof(int) * (size_t)h->nb);
+    int* place = nullptr;
+    if (!d.brec || !d.sopp ||
+        cudaMallocAsync((void**)&place, sizeof(int) * (size_t)h->nb, h->stream) != cudaSuccess) {
+      cudaGetLastError();
+      h->err.clear();
+      h->no_records = true;
+      return 0;
+    }
+    k_sorted_place<<<G, T, 0, h->stream>>>(h->nb, d.sbond, place);
+    LPM_LAUNCHED(h, "k_sorted_place");
+    k_sorted_opp<<<G, T, 0, h->stream>>>(h->nb, d.sbond, d.opp, place, d.sopp);
+    LPM_LAUNCHED(h, "k_sorted_opp");
+    LPM_CUDA(h, cudaFreeAsync(place, h->stream));
+  }
+  k_bond_records<<<G, T, 0, h->stream>>>(h->nb, d.sbond, d.cs, d.Tv, d.bdamage, (double2*)d.brec);
+  LPM_LAUNCHED(h, "k_bond_records");
+  return 1;
+}
+
 int launch_assemble(lpm_handle* h, int tangent, int bc) {
   if (h->mf) return mf_assemble(h, tangent, bc);
   Dev& d = h->d;
@@ -433,15 +502,21 @@ int launch_assemble(lpm_handle* h, int tangent, int bc) {
     // padding slots stay zero for the life of the handle
     LPM_CUDA(h, cudaMemsetAsync(d.A64, 0, sizeof(double) * std::max<size_t>(vals, 1), h->stream));
   }
+  const int ra = bond_records(h);
+  if (ra < 0) return ra;
   AsmView v{d.bptr, d.lptr, d.sell_ptr, d.scol, d.rowlen, d.sbond, d.sp2, d.opp, d.cs, d.cs_sum, d.tsum, d.msum,
-            d.Kn, d.Tv, d.bdamage, d.A64, h->nslots, h->n, h->nslice, tangent == LPM_TANGENT_SYMMETRIC ? 1 : 0};
+            d.Kn, d.Tv, d.bdamage, (const double2*)d.brec, d.sopp, d.A64, h->nslots, h->n, h->nslice,
+            tangent == LPM_TANGENT_SYMMETRIC ? 1 : 0};
   const int T = 256;
   const int G = grid_for((long long)h->nslice * 32, T, 152 * 64);
-  if (dim == 3)
-    k_assemble<3><<<G, T, 0, h->stream>>>(v);
-  else
-    k_assemble<2><<<G, T, 0, h->stream>>>(v);
-  LPM_LAUNCHED(h, "k_assemble");
+  {
+    const int TA = 32 * std::min(kAsmThreads / 32, std::max(1, (h->maxw + kVec - 1) / kVec));
+    if (dim == 3)
+      (ra ? k_assemble<3, true> : k_assemble<3, false>)<<<h->nslice, TA, 0, h->stream>>>(v);
+    else
+      (ra ? k_assemble<2, true> : k_assemble<2, false>)<<<h->nslice, TA, 0, h->stream>>>(v);
+    LPM_LAUNCHED(h, "k_assemble");
+  }
   if (bc == LPM_BC_ELIMINATE) {
     const int GR = grid_for(h->n, kRedThreads, kMaxRedBlocks);
     if (dim == 3)
