@@ -65,13 +65,16 @@ __global__ void k_jac_prep(int n, const int64_t* __restrict__ bptr, const int64_
                            const double* __restrict__ bforce, const double* __restrict__ Kn,
                            const double* __restrict__ Tv, int* __restrict__ jp2, int* __restrict__ jopp,
                            int* __restrict__ jlayer, double* __restrict__ jc, double* __restrict__ jk,
-                           double* __restrict__ jt, double* __restrict__ jf, int64_t nslot) {
+                           double* __restrict__ jt, double* __restrict__ jf, unsigned* __restrict__ jq,
+                           double* __restrict__ jg, double* __restrict__ jo, double* __restrict__ jT,
+                           int64_t nslot) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int sl = i / 32;
   const int len = (int)((jbase[sl + 1] - jbase[sl]) / 32);
   const int64_t s0 = jbase[sl] + (i % 32);
   const int nb = (int)(bptr[i + 1] - bptr[i]);
+  double T[NL][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
   for (int k = 0; k < len; ++k) {
     const int64_t s = s0 + 32 * (int64_t)k;
     if (k < nb && !is_broken(bdamage[bptr[i] + k])) {
@@ -85,14 +88,28 @@ __global__ void k_jac_prep(int n, const int64_t* __restrict__ bptr, const int64_
       jc[2 * nslot + s] = cs[3 * b + 2];
       jk[s] = 2.0 * w * Kn[b];
       jt[s] = 2.0 * w * Tv[b];
-      jf[s] = 0.5 * (bforce[b] + bforce[opp[b]]) / dis[b];
+      const int o = opp[b];
+      const double rf = 0.5 * (bforce[b] + bforce[o]) / dis[b], t = w * Tv[b];
+      jf[s] = rf;
+      const double wo = is_broken(bdamage[o]) ? 0.0 : 1.0 - bdamage[o];
+      jq[s] = (unsigned)bp2[b] | (blayer[b] ? 1u << 31 : 0u);
+      jg[s] = (w * Kn[b] + wo * Kn[o]) - rf;
+      jo[s] = wo * Tv[o];
+#pragma unroll
+      for (int e = 0; e < 3; ++e) (blayer[b] ? T[1] : T[0])[e] += t * cs[3 * b + e];
     } else {
       jp2[s] = i;
       jopp[s] = (int)s;
       jlayer[s] = 0;
       jc[s] = jc[nslot + s] = jc[2 * nslot + s] = 0.0;
-      jk[s] = jt[s] = jf[s] = 0.0;
+      jk[s] = jt[s] = jf[s] = jg[s] = jo[s] = 0.0;
+      jq[s] = (unsigned)i;
     }
+  }
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    jT[6 * (int64_t)i + e] = T[0][e];
+    jT[6 * (int64_t)i + 3 + e] = T[1][e];
   }
 }
 
@@ -107,14 +124,105 @@ struct JacView {
   const double* __restrict__ jf;
   double* __restrict__ jd;  // d dLe, then d f, per slot
   int64_t nslot;
+  // the product alone (jvp_*): partner and layer (top bit), the constants g
+  // and o of a slot, T of a particle's layers, and the sums d D_i^l
+  const unsigned* __restrict__ jq;
+  const double* __restrict__ jg;
+  const double* __restrict__ jo;
+  const double* __restrict__ jT;
+  double* __restrict__ jD;
 };
+
+// The product H v alone, with no other change of the bonds.  A bond and its
+// opposite stretch alike (d dLe_b = c_b . u_b, u_b = v_i - v_j, is the same
+// from both ends), so
+//   d Pin_i = sum_b [ rf_b u_b + c_b (g_b d dLe_b + o_b d D_j^l) ] + sum_l T_i^l d D_i^l,
+// with rf = F/dis, g = w Kn + w' Kn' - rf (primes: the opposite bond, 0 when
+// it is broken), o = w' Tv' and T_i^l = sum w Tv c.  The first pass makes only
+// the sums d D, the second the rest; no value per bond passes between them.
+// Bound by the FP64 pipe (6 and 14 operations a slot; 40 us at 41^3 particles)
+// and by 28 and 52 bytes a slot from L2.  k_jvp_bonds and k_jvp_particles,
+// which hand d f from pass to pass, take 28 operations and 132 bytes: a
+// gradient at 41^3 particles (255 iterations) 33.4 ms with them, 22.5 with these;
+// they stay where the bonds change otherwise too.
+template <int DIM>
+__device__ __forceinline__ void load_u(const double* __restrict__ v, const double (&vi)[DIM], int j, double (&u)[DIM]) {
+#pragma unroll
+  for (int k = 0; k < DIM; ++k) u[k] = vi[k] - __ldg(&v[(int64_t)DIM * j + k]);
+}
+template <int DIM>
+__global__ void __launch_bounds__(128) k_jvp_sums(int n, JacView J, const double* __restrict__ v, const CgScalars* cg) {
+  if (cg && cg->done) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t s0 = J.jbase[i / 32] + (i % 32), s1 = J.jbase[i / 32 + 1];
+  double vi[DIM];
+#pragma unroll
+  for (int k = 0; k < DIM; ++k) vi[k] = v[(int64_t)DIM * i + k];
+  double dD0 = 0.0, dD1 = 0.0;
+#pragma unroll 3
+  for (int64_t s = s0; s < s1; s += 32) {
+    const unsigned q = __ldg(&J.jq[s]);
+    double u[DIM], D = q >> 31 ? dD1 : dD0;
+    load_u<DIM>(v, vi, (int)(q & 0x7fffffffu), u);
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) D = fma(__ldg(&J.jc[k * J.nslot + s]), u[k], D);
+    if (q >> 31)
+      dD1 = D;
+    else
+      dD0 = D;
+  }
+  reinterpret_cast<double2*>(J.jD)[i] = make_double2(dD0, dD1);
+}
+// With `cg` also p.q over the grid and, in the last block, alpha.
+template <int DIM>
+__global__ void __launch_bounds__(128) k_jvp_forces(int n, JacView J, const double* __restrict__ v,
+                                                    const int* __restrict__ mask, double* __restrict__ y,
+                                                    CgScalars* cg, double* partials, unsigned int* ticket) {
+  if (cg && cg->done) return;
+  double acc = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int64_t s0 = J.jbase[i / 32] + (i % 32), s1 = J.jbase[i / 32 + 1];
+    double vi[DIM], P[DIM];
+    const double2 D = reinterpret_cast<const double2*>(J.jD)[i];
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) {
+      vi[k] = v[(int64_t)DIM * i + k];
+      P[k] = fma(J.jT[6 * (int64_t)i + k], D.x, J.jT[6 * (int64_t)i + 3 + k] * D.y);
+    }
+#pragma unroll 3
+    for (int64_t s = s0; s < s1; s += 32) {
+      const unsigned q = __ldg(&J.jq[s]);
+      const int j = (int)(q & 0x7fffffffu);
+      double u[DIM], c[DIM], dd = 0.0;
+      load_u<DIM>(v, vi, j, u);
+#pragma unroll
+      for (int k = 0; k < DIM; ++k) {
+        c[k] = __ldg(&J.jc[k * J.nslot + s]);
+        dd = fma(c[k], u[k], dd);
+      }
+      const double g = fma(__ldg(&J.jg[s]), dd, __ldg(&J.jo[s]) * __ldg(&J.jD[2 * (int64_t)j + (q >> 31)]));
+      const double rf = __ldg(&J.jf[s]);
+#pragma unroll
+      for (int k = 0; k < DIM; ++k) P[k] = fma(c[k], g, fma(rf, u[k], P[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) {
+      const double yk = (mask && mask[3 * i + k]) ? 0.0 : P[k];
+      y[(int64_t)DIM * i + k] = yk;
+      acc += vi[k] * yk;
+    }
+  }
+  if (!cg) return;
+  double w[1] = {acc}, tot[1];
+  if (grid_sum<1>(w, partials, ticket, tot) && threadIdx.x == 0) cg->alpha = cg->abs_new / tot[0];
+}
 
 // Pass 1 of H v: d dLe per slot and the per-layer sums d D_i^l, then d f.
 // With dlp (per slot) the plastic stretches move too: d dLe -= d dLp; with
 // dfk (per slot) the bond constants too: d f += dfk.
 __global__ void k_jvp_bonds(int n, int dim, JacView J, const double* __restrict__ v, const double* __restrict__ dlp,
-                            const double* __restrict__ dfk, const CgScalars* cg) {
-  if (cg && cg->done) return;
+                            const double* __restrict__ dfk) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int sl = i / 32;
@@ -143,13 +251,9 @@ __global__ void k_jvp_bonds(int n, int dim, JacView J, const double* __restrict_
 }
 
 // Pass 2 of H v: y_i = d Pin_i (zero on constrained DOFs when `mask` is
-// given).  With `cg` set it also forms p.q over the grid and, in the last
-// block, alpha = (r.z) / (p.q) for the CG update.
+// given).
 __global__ void __launch_bounds__(256) k_jvp_particles(int n, int dim, JacView J, const double* __restrict__ v,
-                                                       const int* __restrict__ mask, double* __restrict__ y,
-                                                       CgScalars* cg, double* partials, unsigned int* ticket) {
-  if (cg && cg->done) return;
-  double acc = 0.0;
+                                                       const int* __restrict__ mask, double* __restrict__ y) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int sl = i / 32;
     const int len = (int)((J.jbase[sl + 1] - J.jbase[sl]) / 32);
@@ -174,14 +278,9 @@ __global__ void __launch_bounds__(256) k_jvp_particles(int n, int dim, JacView J
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       if (k >= dim) break;
-      const double yk = (mask && mask[3 * i + k]) ? 0.0 : P[k];
-      y[(int64_t)dim * i + k] = yk;
-      acc += vi[k] * yk;
+      y[(int64_t)dim * i + k] = (mask && mask[3 * i + k]) ? 0.0 : P[k];
     }
   }
-  if (!cg) return;
-  double w[1] = {acc}, tot[1];
-  if (grid_sum<1>(w, partials, ticket, tot) && threadIdx.x == 0) cg->alpha = cg->abs_new / tot[0];
 }
 
 // Exact diagonal of H (one DOF of particle i moved, its partners' layer sums
@@ -549,7 +648,13 @@ static int jacobian_prepare(lpm_handle* h) {
     d.jt = (double*)dev_alloc(h, sizeof(double) * S);
     d.jf = (double*)dev_alloc(h, sizeof(double) * S);
     d.jd = (double*)dev_alloc(h, sizeof(double) * S);
-    if (!d.jbase || !d.jslot_of || !d.jp2 || !d.jopp || !d.jlayer || !d.jc || !d.jk || !d.jt || !d.jf || !d.jd)
+    d.jq = (unsigned*)dev_alloc(h, sizeof(unsigned) * S);
+    d.jg = (double*)dev_alloc(h, sizeof(double) * S);
+    d.jo = (double*)dev_alloc(h, sizeof(double) * S);
+    d.jT = (double*)dev_alloc(h, sizeof(double) * 6 * (size_t)std::max(n, 1));
+    d.jD = (double*)dev_alloc(h, sizeof(double) * 2 * (size_t)std::max(n, 1));
+    if (!d.jbase || !d.jslot_of || !d.jp2 || !d.jopp || !d.jlayer || !d.jc || !d.jk || !d.jt || !d.jf || !d.jd ||
+        !d.jq || !d.jg || !d.jo || !d.jT || !d.jD)
       return LPM_ERR_NOMEM;
     LPM_CUDA(h, cudaMemcpy(d.jbase, jb.data(), sizeof(int64_t) * jb.size(), cudaMemcpyHostToDevice));
     k_jac_slots<<<grid_for(n, 128), 128, 0, h->stream>>>(n, d.bptr, d.jbase, d.jslot_of);
@@ -557,9 +662,14 @@ static int jacobian_prepare(lpm_handle* h) {
   }
   k_jac_prep<<<grid_for(n, 128), 128, 0, h->stream>>>(n, d.bptr, d.jbase, d.jslot_of, d.bp2, d.blayer, d.opp, d.cs,
                                                       d.dis, d.bdamage, d.bforce, d.Kn, d.Tv, d.jp2, d.jopp,
-                                                      d.jlayer, d.jc, d.jk, d.jt, d.jf, h->jslots);
+                                                      d.jlayer, d.jc, d.jk, d.jt, d.jf, d.jq, d.jg, d.jo, d.jT, h->jslots);
   LPM_LAUNCHED(h, "k_jac_prep");
   return LPM_OK;
+}
+
+static JacView jac_view(const lpm_handle* h) {
+  const Dev& d = h->d;
+  return JacView{d.jbase, d.jp2, d.jopp, d.jlayer, d.jc, d.jk, d.jt, d.jf, d.jd, h->jslots, d.jq, d.jg, d.jo, d.jT, d.jD};
 }
 
 // y = H v (mask: zero the constrained rows); with cg, p.q and alpha too;
@@ -567,12 +677,26 @@ static int jacobian_prepare(lpm_handle* h) {
 static int apply_jacobian(lpm_handle* h, const double* v, double* y, bool masked, CgScalars* cg,
                           const double* dlp = nullptr, const double* dfk = nullptr) {
   Dev& d = h->d;
-  const JacView J{d.jbase, d.jp2, d.jopp, d.jlayer, d.jc, d.jk, d.jt, d.jf, d.jd, h->jslots};
-  k_jvp_bonds<<<grid_for(h->n, 128), 128, 0, h->stream>>>(h->n, h->dim, J, v, dlp, dfk, cg);
-  LPM_LAUNCHED(h, "k_jvp_bonds");
-  k_jvp_particles<<<grid_for(h->n, 256, kMaxRedBlocks), 256, 0, h->stream>>>(
-      h->n, h->dim, J, v, masked ? d.mask : nullptr, y, cg, d.red.partials, d.red.ticket + 8);
-  LPM_LAUNCHED(h, "k_jvp_particles");
+  const JacView J = jac_view(h);
+  const int* mask = masked ? d.mask : nullptr;
+  if (dlp || dfk) {
+    k_jvp_bonds<<<grid_for(h->n, 128), 128, 0, h->stream>>>(h->n, h->dim, J, v, dlp, dfk);
+    LPM_LAUNCHED(h, "k_jvp_bonds");
+    k_jvp_particles<<<grid_for(h->n, 256, kMaxRedBlocks), 256, 0, h->stream>>>(h->n, h->dim, J, v, mask, y);
+    LPM_LAUNCHED(h, "k_jvp_particles");
+    return LPM_OK;
+  }
+  const int T = 128, G1 = grid_for(h->n, T), G2 = grid_for(h->n, T, kMaxRedBlocks);
+  if (h->dim == 3)
+    k_jvp_sums<3><<<G1, T, 0, h->stream>>>(h->n, J, v, cg);
+  else
+    k_jvp_sums<2><<<G1, T, 0, h->stream>>>(h->n, J, v, cg);
+  LPM_LAUNCHED(h, "k_jvp_sums");
+  if (h->dim == 3)
+    k_jvp_forces<3><<<G2, T, 0, h->stream>>>(h->n, J, v, mask, y, cg, d.red.partials, d.red.ticket + 8);
+  else
+    k_jvp_forces<2><<<G2, T, 0, h->stream>>>(h->n, J, v, mask, y, cg, d.red.partials, d.red.ticket + 8);
+  LPM_LAUNCHED(h, "k_jvp_forces");
   return LPM_OK;
 }
 
@@ -596,7 +720,9 @@ static int jacobian_cg(lpm_handle* h, const double* g, double* x, double tol, lo
                                                             d.bdamage, d.bforce, d.Kn, d.Tv, d.mask, d.adj_invd);
   LPM_LAUNCHED(h, "k_jac_invdiag");
   if (maxit < 0) maxit = 2LL * m;
-  const int GV = grid_for(m, 256, kMaxRedBlocks);
+  // two blocks per SM: the fold over the blocks of all of a 41^3 cube's DOFs
+  // took 4 us of an iteration more
+  const int GV = grid_for(m, 256, h->sms > 0 ? std::min(2 * h->sms, kMaxRedBlocks) : kMaxRedBlocks);
   k_cg_init<double><<<GV, 256, 0, h->stream>>>(m, g, x, d.adj_r, d.adj_p, d.adj_invd, d.cg, tol, maxit,
                                                d.red.partials, d.red.ticket + 2);
   LPM_LAUNCHED(h, "k_cg_init");
@@ -1029,7 +1155,7 @@ int tangent_step(lpm_handle* h) {
     if (!d.tg_jdl || !d.tg_jdk) return LPM_ERR_NOMEM;
   }
   LPM_CUDA(h, cudaMemsetAsync(d.adj_a, 0, sizeof(double) * m, h->stream));  // a zero position change
-  const JacView J{d.jbase, d.jp2, d.jopp, d.jlayer, d.jc, d.jk, d.jt, d.jf, d.jd, h->jslots};
+  const JacView J = jac_view(h);
   for (int k = 0; k < h->tg_ndir; ++k) {
     double* tdlp = d.tg_dlp + (size_t)k * std::max<int64_t>(h->nb, 1);
     double* tsv = d.tg_sv + (size_t)k * n * h->nstate;

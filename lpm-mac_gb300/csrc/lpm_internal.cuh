@@ -178,6 +178,8 @@ struct Dev {
   // adjoint: sliced bond data of the exact Jacobian (32 particles per slice)
   int64_t* jbase;
   int *jslot_of, *jp2, *jopp, *jlayer;
+  unsigned* jq;             // the exact Jacobian's product: partner and layer of a slot,
+  double *jg, *jo, *jT, *jD;  // its constants, the particles' sums (lpm_adjoint.cu)
   double *jc, *jk, *jt, *jf, *jd;
   // tangent-linear sensitivity (lpm_tangent_begin): per direction the
   // tangents of dLp [nb], of the state variables [n * nstate], of the
