@@ -110,6 +110,9 @@ int lpm_num_blocks(const lpm_handle* h, int64_t* nblocks);
  * blayer[Nb], opp[Nb] (the opposite bond found by particle.h:207-209). */
 int lpm_get_pattern(const lpm_handle* h, int64_t* cptr, int* cidx);
 int lpm_get_bonds(const lpm_handle* h, int64_t* bptr, int* bp2, int* blayer, int64_t* opp);
+/* The input index of each stored bond (stored order is by owner, then layer,
+ * input order within): order[Nb]. */
+int lpm_get_bond_order(const lpm_handle* h, int64_t* order);
 
 /* Field transfer (host <-> device), sizes as listed with the field ids. */
 int lpm_upload(lpm_handle* h, int field, const double* src);

@@ -111,6 +111,7 @@ def load(build_if_needed=True):
         "lpm_num_blocks": [H, i64p],
         "lpm_get_pattern": [H, i64p, ip],
         "lpm_get_bonds": [H, i64p, ip, ip, i64p],
+        "lpm_get_bond_order": [H, i64p],
         "lpm_upload": [H, ctypes.c_int, dp],
         "lpm_download": [H, ctypes.c_int, dp],
         "lpm_set_mask": [H, ip],
@@ -174,7 +175,7 @@ def load(build_if_needed=True):
 def exported_symbols():
     """Names of the C-ABI entry points this binding uses."""
     return ["lpm_set_device", "lpm_create", "lpm_destroy", "lpm_last_error", "lpm_num_bonds", "lpm_num_blocks", "lpm_get_pattern",
-            "lpm_get_bonds", "lpm_upload", "lpm_download", "lpm_set_mask", "lpm_get_mask", "lpm_set_law",
+            "lpm_get_bonds", "lpm_get_bond_order", "lpm_upload", "lpm_download", "lpm_set_mask", "lpm_get_mask", "lpm_set_law",
             "lpm_update_damage", "lpm_set_types", "lpm_set_nonlocal", "lpm_update_state", "lpm_fatigue_damage",
             "lpm_add_group", "lpm_apply_disp_bc", "lpm_apply_force_bc",
             "lpm_update_geometry_force", "lpm_residual", "lpm_assemble", "lpm_get_K", "lpm_set_operator",
@@ -298,7 +299,8 @@ class Lattice:
         self.ndof = self.dim * self.n
         # input index of each stored bond: stored order is by owner, then
         # layer, input order within (stable)
-        self.bond_perm = np.lexsort((layer, p1))
+        self.bond_perm = np.empty(self.nb, np.int64)
+        self._check(L.lpm_get_bond_order(h, _l(self.bond_perm)))
 
     def close(self):
         if getattr(self, "h", None):

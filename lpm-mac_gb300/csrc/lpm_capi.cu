@@ -70,6 +70,44 @@ T* zeros_new(lpm_handle* h, size_t count) {
   return p;
 }
 
+// Arrays laid out one after the other in one zeroed allocation.
+struct Slab {
+  struct Part {
+    void** p;
+    size_t at;
+  };
+  std::vector<Part> parts;
+  size_t bytes = 0;
+  template <typename T>
+  void add(T** p, size_t count) {
+    parts.push_back({(void**)p, bytes});
+    bytes += (sizeof(T) * std::max<size_t>(count, 1) + 255) / 256 * 256;
+  }
+  int make(lpm_handle* h) {
+    char* base = (char*)dev_alloc(h, bytes);
+    if (!base) return LPM_ERR_NOMEM;
+    LPM_CUDA(h, cudaMemsetAsync(base, 0, bytes, h->stream));
+    for (const Part& q : parts) *q.p = base + q.at;
+    return LPM_OK;
+  }
+};
+
+// Whether every bond has one of its partner, in the same layer, that points
+// back (ids and layers in range).
+bool has_opposites(int n, int64_t nb, const int* p1, const int* p2, const int* layer) {
+  std::vector<int64_t> ptr((size_t)n * NL + 1, 0);
+  for (int64_t b = 0; b < nb; ++b) ptr[(size_t)p1[b] * NL + layer[b] + 1]++;
+  for (size_t k = 1; k < ptr.size(); ++k) ptr[k] += ptr[k - 1];
+  std::vector<int> to((size_t)nb);
+  std::vector<int64_t> at(ptr.begin(), ptr.end() - 1);
+  for (int64_t b = 0; b < nb; ++b) to[(size_t)at[(size_t)p1[b] * NL + layer[b]]++] = p2[b];
+  for (int64_t b = 0; b < nb; ++b) {
+    const size_t k = (size_t)p2[b] * NL + layer[b];
+    if (std::find(to.begin() + ptr[k], to.begin() + ptr[k + 1], p1[b]) == to.begin() + ptr[k + 1]) return false;
+  }
+  return true;
+}
+
 struct FieldRef {
   double* ptr;
   size_t count;
@@ -137,49 +175,6 @@ int lpm_create(int dim, int n, int64_t nb, const double* xyz, const int* p1, con
     if (p1[b] < 0 || p1[b] >= n || p2[b] < 0 || p2[b] >= n || layer[b] < 0 || layer[b] >= NL)
       return arg_error(nullptr, "bond with particle id or layer out of range");
   const size_t N = (size_t)n, B = (size_t)nb;
-  // bond CSR by (p1, layer), stable (bond_layers order)
-  std::vector<int64_t> cnt(N * NL + 1, 0);
-  for (int64_t b = 0; b < nb; ++b) cnt[(size_t)p1[b] * NL + layer[b] + 1]++;
-  for (size_t k = 1; k < cnt.size(); ++k) cnt[k] += cnt[k - 1];
-  std::vector<int64_t> src(B);
-  {
-    std::vector<int64_t> pos(cnt.begin(), cnt.end() - 1);
-    for (int64_t b = 0; b < nb; ++b) src[(size_t)pos[(size_t)p1[b] * NL + layer[b]]++] = b;
-  }
-  std::vector<int64_t> bptr(N + 1), lptr(N);
-  for (size_t i = 0; i <= N; ++i) bptr[i] = cnt[i * NL];
-  for (size_t i = 0; i < N; ++i) lptr[i] = cnt[i * NL + 1];
-  std::vector<int> bp2(B), bl(B), nbonds(N), opp(B, -1);
-  std::vector<double> kn(B), tv(B), dis0(B);
-  for (size_t b = 0; b < B; ++b) {
-    bp2[b] = p2[src[b]];
-    bl[b] = layer[src[b]];
-    kn[b] = Kn[src[b]];
-    tv[b] = Tv[src[b]];
-  }
-  for (size_t i = 0; i < N; ++i) {
-    nbonds[i] = (int)(bptr[i + 1] - bptr[i]);
-    for (int64_t b = bptr[i]; b < bptr[i + 1]; ++b) {
-      const double* xi = xyz + 3 * i;
-      const double* xj = xyz + 3 * (size_t)bp2[(size_t)b];
-      const double dx = xi[0] - xj[0], dy = xi[1] - xj[1], dz = xi[2] - xj[2];
-      dis0[(size_t)b] = std::sqrt(dx * dx + dy * dy + dz * dz);
-      // opposite bond: the first bond of p2 in the same layer pointing back
-      // (particle.h:207-209)
-      const int j = bp2[(size_t)b], l = bl[(size_t)b];
-      const int64_t jb = l == 0 ? bptr[(size_t)j] : lptr[(size_t)j];
-      const int64_t je = l == 0 ? lptr[(size_t)j] : bptr[(size_t)j + 1];
-      for (int64_t c = jb; c < je; ++c)
-        if (bp2[(size_t)c] == (int)i) {
-          opp[(size_t)b] = (int)c;
-          break;
-        }
-      if (opp[(size_t)b] < 0) {
-        g_err = "bond without an opposite bond in the same layer";
-        return LPM_ERR_TOPOLOGY;
-      }
-    }
-  }
   lpm_handle* h = new lpm_handle();
   h->dim = dim;
   h->n = n;
@@ -187,70 +182,65 @@ int lpm_create(int dim, int n, int64_t nb, const double* xyz, const int* p1, con
   h->particle_volume = particle_volume;
   h->nneighbors = nneighbors;
   cudaGetDevice(&h->device);
-  cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-  if (e != cudaSuccess) {
-    int st = cuda_fail(h, e, "cudaStreamCreate");
-    delete h;
-    return st;
-  }
   auto fail = [&](int st) {
     g_err = h->err;
     lpm_destroy(h);
+    // without a device or its memory a list that is no topology is refused as one all the same
+    if (st != LPM_ERR_TOPOLOGY && !has_opposites(n, nb, p1, p2, layer)) {
+      g_err = kNoOpposite;
+      return (int)LPM_ERR_TOPOLOGY;
+    }
     return st;
   };
-  // partner-sorted view of each (particle, layer) bond segment, used by the
-  // tangent's common-neighbour merge
-  std::vector<int> sbond(B), sp2(B);
-  for (size_t i = 0; i < N; ++i)
-    for (int l = 0; l < NL; ++l) {
-      const int64_t b0 = l == 0 ? bptr[i] : lptr[i], b1 = l == 0 ? lptr[i] : bptr[i + 1];
-      for (int64_t b = b0; b < b1; ++b) sbond[(size_t)b] = (int)b;
-      std::stable_sort(sbond.begin() + b0, sbond.begin() + b1,
-                       [&](int a, int c) { return bp2[(size_t)a] < bp2[(size_t)c]; });
-      for (int64_t b = b0; b < b1; ++b) sp2[(size_t)b] = bp2[(size_t)sbond[(size_t)b]];
-    }
+  cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
+  if (e != cudaSuccess) {
+    h->stream = nullptr;
+    return fail(cuda_fail(h, e, "cudaStreamCreate"));
+  }
+  // every array of the handle's life in one allocation, zeroed by one fill
+  // (an allocation and a fill each took 60 us an array)
   Dev& d = h->d;
-  bool ok = true;
-  ok = ok && (d.sbond = upload_new(h, sbond.data(), B)) && (d.sp2 = upload_new(h, sp2.data(), B)) &&
-       (d.tsum = zeros_new<double>(h, NL * 3 * N)) && (d.msum = zeros_new<double>(h, NL * 6 * N));
-  ok = ok && (d.x = upload_new(h, xyz, 3 * N)) && (d.x0 = upload_new(h, xyz, 3 * N)) &&
-       (d.xlast = upload_new(h, xyz, 3 * N));
-  ok = ok && (d.pin = zeros_new<double>(h, 3 * N)) && (d.pex = zeros_new<double>(h, 3 * N)) &&
-       (d.stress = zeros_new<double>(h, 6 * N)) && (d.dvis = zeros_new<double>(h, N)) &&
-       (d.dle_tot = zeros_new<double>(h, NL * N)) && (d.tdle_tot = zeros_new<double>(h, NL * N)) &&
-       (d.cs_sum = zeros_new<double>(h, NL * 3 * N)) && (d.damage = zeros_new<double>(h, N)) &&
-       (d.damage_last = zeros_new<double>(h, N)) && (d.mask = zeros_new<int>(h, 3 * N)) &&
-       (d.nbonds = upload_new(h, nbonds.data(), N)) && (d.fixed = zeros_new<unsigned char>(h, 3 * N));
-  ok = ok && (d.bptr = upload_new(h, bptr.data(), N + 1)) && (d.lptr = upload_new(h, lptr.data(), N)) &&
-       (d.bp2 = upload_new(h, bp2.data(), B)) && (d.blayer = upload_new(h, bl.data(), B)) &&
-       (d.opp = upload_new(h, opp.data(), B)) && (d.Kn = upload_new(h, kn.data(), B)) &&
-       (d.Tv = upload_new(h, tv.data(), B)) && (d.dis0 = upload_new(h, dis0.data(), B)) &&
-       (d.dis = upload_new(h, dis0.data(), B)) && (d.dis_last = upload_new(h, dis0.data(), B));
-  ok = ok && (d.dLe = zeros_new<double>(h, B)) && (d.dLp = zeros_new<double>(h, B)) &&
-       (d.dLp_last = zeros_new<double>(h, B)) && (d.bstrain = zeros_new<double>(h, B)) &&
-       (d.cs = zeros_new<double>(h, 3 * B)) && (d.bforce = zeros_new<double>(h, B)) &&
-       (d.bforce_last = zeros_new<double>(h, B)) && (d.bdamage = zeros_new<double>(h, B)) &&
-       (d.bdamage_last = zeros_new<double>(h, B));
   const size_t ndof = (size_t)dim * N;
-  ok = ok && (d.rhs = zeros_new<double>(h, ndof)) && (d.disp = zeros_new<double>(h, ndof)) &&
-       (d.x64 = zeros_new<double>(h, ndof)) && (d.r64 = zeros_new<double>(h, ndof)) &&
-       (d.p64 = zeros_new<double>(h, ndof)) && (d.q64 = zeros_new<double>(h, ndof)) &&
-       (d.invd64 = zeros_new<double>(h, ndof));
-  ok = ok && (d.red.partials = zeros_new<double>(h, (size_t)kMaxRedBlocks * 4)) &&
-       (d.red.ticket = zeros_new<unsigned int>(h, 16)) && (d.cg = zeros_new<CgScalars>(h, 1)) &&
-       (d.norms = zeros_new<double>(h, 8)) && (d.gbar = zeros_new<unsigned long long>(h, 1));
-  std::vector<double> crit(N, 1.0);
-  ok = ok && (d.crit = upload_new(h, crit.data(), N)) && (d.pp = upload_new(h, crit.data(), N)) &&
-       (d.ptype = zeros_new<int>(h, N)) && (d.state = zeros_new<double>(h, N)) &&
-       (d.state_last = zeros_new<double>(h, N)) && (d.ddot_local = zeros_new<double>(h, N)) &&
-       (d.ddot_nl = zeros_new<double>(h, N)) && (d.nonlocal_L = zeros_new<double>(h, N));
-  if (!ok) return fail(h->err.empty() ? LPM_ERR_CUDA : LPM_ERR_NOMEM);
+  Slab slab;
+  for (double** p : {&d.x, &d.x0, &d.xlast, &d.pin, &d.pex}) slab.add(p, 3 * N);
+  for (double** p : {&d.stress, &d.tsum, &d.cs_sum}) slab.add(p, 6 * N);
+  slab.add(&d.msum, NL * 6 * N);
+  for (double** p : {&d.dle_tot, &d.tdle_tot}) slab.add(p, NL * N);
+  for (double** p : {&d.dvis, &d.damage, &d.damage_last, &d.crit, &d.pp, &d.state, &d.state_last, &d.ddot_local,
+                     &d.ddot_nl, &d.nonlocal_L})
+    slab.add(p, N);
+  for (double** p : {&d.Kn, &d.Tv, &d.dis0, &d.dis, &d.dis_last, &d.dLe, &d.dLp, &d.dLp_last, &d.bstrain, &d.bforce,
+                     &d.bforce_last, &d.bdamage, &d.bdamage_last})
+    slab.add(p, B);
+  slab.add(&d.cs, 3 * B);
+  for (double** p : {&d.rhs, &d.disp, &d.x64, &d.r64, &d.p64, &d.q64, &d.invd64}) slab.add(p, ndof);
+  slab.add(&d.red.partials, (size_t)kMaxRedBlocks * 4);
+  slab.add(&d.norms, 8);
+  slab.add(&d.cg, 1);
+  slab.add(&d.gbar, 1);
+  slab.add(&d.red.ticket, 16);
+  slab.add(&d.bptr, N + 1);
+  slab.add(&d.lptr, N);
+  for (int** p : {&d.bp2, &d.blayer, &d.opp, &d.sbond, &d.sp2, &d.bsrc}) slab.add(p, B);
+  for (int** p : {&d.nbonds, &d.ptype}) slab.add(p, N);
+  slab.add(&d.mask, 3 * N);
+  slab.add(&d.fixed, 3 * N);
+  int st = slab.make(h);
+  if (st) return fail(st);
+  if (cudaMemcpyAsync(d.x, xyz, sizeof(double) * 3 * N, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+      cudaMemcpyAsync(d.x0, d.x, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess ||
+      cudaMemcpyAsync(d.xlast, d.x, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess) {
+    h->err = "lpm_create: copy of the coordinates failed";
+    return fail(LPM_ERR_CUDA);
+  }
+  st = build_bonds(h, p1, p2, layer, Kn, Tv);
+  if (st) return fail(st);
   if (cudaMallocHost((void**)&h->h_cg, sizeof(CgScalars)) != cudaSuccess ||
       cudaMallocHost((void**)&h->h_norms, 8 * sizeof(double)) != cudaSuccess) {
     h->err = "cudaMallocHost failed";
     return fail(LPM_ERR_NOMEM);
   }
-  int st = build_pattern(h);
+  st = build_pattern(h);
   if (st) return fail(st);
   *out = h;
   return LPM_OK;
@@ -291,6 +281,15 @@ int lpm_get_pattern(const lpm_handle* h, int64_t* cptr, int* cidx) {
   lpm_handle* hh = const_cast<lpm_handle*>(h);
   if (cptr) LPM_CUDA(hh, cudaMemcpy(cptr, h->d.cptr, sizeof(int64_t) * (h->n + 1), cudaMemcpyDeviceToHost));
   if (cidx) LPM_CUDA(hh, cudaMemcpy(cidx, h->d.cidx, sizeof(int) * h->nblk, cudaMemcpyDeviceToHost));
+  return LPM_OK;
+}
+
+int lpm_get_bond_order(const lpm_handle* h, int64_t* order) {
+  if (!h || !order) return LPM_ERR_ARG;
+  lpm_handle* hh = const_cast<lpm_handle*>(h);
+  std::vector<int> o((size_t)h->nb);
+  LPM_CUDA(hh, cudaMemcpy(o.data(), h->d.bsrc, sizeof(int) * h->nb, cudaMemcpyDeviceToHost));
+  std::copy(o.begin(), o.end(), order);
   return LPM_OK;
 }
 

@@ -110,6 +110,7 @@ struct Dev {
   int *bp2, *blayer, *opp;
   double* brec;  // an assembly's bond records (lpm_tangent.cu)
   int* sopp;
+  int* bsrc;  // input index of each stored bond
   int *sbond, *sp2;  // per (particle, layer) segment: bond ids and partners sorted by partner id
   double *Kn, *Tv, *dis0, *dis, *dis_last, *dLe, *dLp, *dLp_last, *bstrain, *cs, *bforce, *bforce_last, *bdamage,
       *bdamage_last;
@@ -315,6 +316,9 @@ int launch_static_damage(lpm_handle* h, int* any_new);
 int launch_fatigue_damage(lpm_handle* h, double dt, int* any_new);
 // pattern / tangent (lpm_tangent.cu)
 int build_pattern(lpm_handle* h);
+// a lattice's bond arrays from the caller's list (lpm_setup.cu)
+inline constexpr const char* kNoOpposite = "bond without an opposite bond in the same layer";
+int build_bonds(lpm_handle* h, const int* p1, const int* p2, const int* layer, const double* Kn, const double* Tv);
 int launch_assemble(lpm_handle* h, int tangent, int bc);
 int convert_A32(lpm_handle* h);
 // matrix-free operator (lpm_mfree.cu): the per-assembly data, the Jacobi
