@@ -38,13 +38,83 @@ __global__ void k_count_candidates(int n, const int64_t* __restrict__ bptr, cons
   cnt[i] = c;
 }
 
-// Candidates of particle i in the reference's push order, then an insertion
-// sort and unique in place.  Writes the unique count.
-__global__ void k_fill_candidates(int n, const int64_t* __restrict__ bptr, const int64_t* __restrict__ lptr,
-                                  const int* __restrict__ bp2, const int64_t* __restrict__ cand_ptr,
-                                  int* __restrict__ cand, int64_t* __restrict__ ucnt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Candidates of particle i, sorted and unique in place; writes their count.
+// Their order before the sort does not matter, so a warp collects them a
+// bond's segment at a time into shared memory and sorts them there
+// (bitonic).  A particle of more candidates than kWarpCand is left to
+// k_fill_candidates_long, one thread's heapsort in global memory.  By one
+// thread's insertion sort in global memory all particles took 4.6 ms of 51^3
+// (198 candidates each), with the warps 0.47.
+constexpr int kWarpCand = 1024, kCandWarps = 4;
+__global__ void __launch_bounds__(32 * kCandWarps) k_fill_candidates(int n, const int64_t* __restrict__ bptr,
+                                                                    const int64_t* __restrict__ lptr,
+                                                                    const int* __restrict__ bp2,
+                                                                    const int* __restrict__ blayer,
+                                                                    const int64_t* __restrict__ cand_ptr,
+                                                                    int* __restrict__ cand,
+                                                                    int64_t* __restrict__ ucnt) {
+  __shared__ int sm[kCandWarps][kWarpCand];
+  const int lane = threadIdx.x & 31, i = blockIdx.x * kCandWarps + (threadIdx.x >> 5);
   if (i >= n) return;
+  const int m = (int)min(cand_ptr[i + 1] - cand_ptr[i], (int64_t)INT_MAX);
+  if (m > kWarpCand) return;
+  int* c = sm[threadIdx.x >> 5];
+  const int64_t b0 = bptr[i], b1 = bptr[i + 1];
+  // 32 bonds at a time: each lane's segment, then its place among them
+  int at = 0;
+  for (int64_t g = b0; g < b1; g += 32) {
+    int64_t kb = 0, ke = 0;
+    int k = 0, len = 0;
+    if (g + lane < b1) {
+      k = bp2[g + lane];
+      layer_range(bptr, lptr, k, blayer[g + lane], kb, ke);
+      len = 1 + (int)(ke - kb);
+    }
+    int s = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += t;
+    }
+    int to = at + s - len;
+    if (len) {
+      c[to++] = k;
+      for (int64_t b = kb; b < ke; ++b) c[to++] = bp2[b];
+    }
+    at += __shfl_sync(0xffffffffu, s, 31);
+  }
+  int M = 32;
+  while (M < m) M *= 2;
+  for (int a = m + lane; a < M; a += 32) c[a] = INT_MAX;
+  __syncwarp();
+  for (int k = 2; k <= M; k *= 2)
+    for (int q = k / 2; q > 0; q /= 2) {
+      for (int t = lane; t < M / 2; t += 32) {
+        const int lo = 2 * q * (t / q) + t % q, hi = lo + q;
+        const int a = c[lo], b = c[hi];
+        if ((a > b) == ((lo & k) == 0)) {
+          c[lo] = b;
+          c[hi] = a;
+        }
+      }
+      __syncwarp();
+    }
+  int* out = cand + cand_ptr[i];
+  int u = 0;
+  for (int a0 = 0; a0 < m; a0 += 32) {
+    const int a = a0 + lane;
+    const bool first = a < m && (a == 0 || c[a] != c[a - 1]);
+    const unsigned mask = __ballot_sync(0xffffffffu, first);
+    if (first) out[u + __popc(mask & ((1u << lane) - 1u))] = c[a];
+    u += __popc(mask);
+  }
+  if (lane == 0) ucnt[i] = u;
+}
+__global__ void k_fill_candidates_long(int n, const int64_t* __restrict__ bptr, const int64_t* __restrict__ lptr,
+                                       const int* __restrict__ bp2, const int64_t* __restrict__ cand_ptr,
+                                       int* __restrict__ cand, int64_t* __restrict__ ucnt) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n || cand_ptr[i + 1] - cand_ptr[i] <= kWarpCand) return;
   int* c = cand + cand_ptr[i];
   int64_t m = 0;
   for (int l = 0; l < NL; ++l) {
@@ -58,14 +128,21 @@ __global__ void k_fill_candidates(int n, const int64_t* __restrict__ bptr, const
       for (int64_t b2 = kb; b2 < ke; ++b2) c[m++] = bp2[b2];
     }
   }
-  for (int64_t a = 1; a < m; ++a) {
-    const int v = c[a];
-    int64_t t = a - 1;
-    while (t >= 0 && c[t] > v) {
-      c[t + 1] = c[t];
-      --t;
+  auto sift = [&](int64_t r, int64_t e) {
+    const int v = c[r];
+    for (int64_t q; (q = 2 * r + 1) < e; r = q) {
+      if (q + 1 < e && c[q] < c[q + 1]) ++q;
+      if (v >= c[q]) break;
+      c[r] = c[q];
     }
-    c[t + 1] = v;
+    c[r] = v;
+  };
+  for (int64_t r = m / 2 - 1; r >= 0; --r) sift(r, m);
+  for (int64_t e = m - 1; e > 0; --e) {
+    const int v = c[0];
+    c[0] = c[e];
+    c[e] = v;
+    sift(0, e);
   }
   int64_t u = 0;
   for (int64_t a = 0; a < m; ++a)
@@ -410,8 +487,13 @@ int build_pattern(lpm_handle* h) {
   LPM_CUDA(h, cudaMemcpyAsync(cand_ptr, hp.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, h->stream));
   int* cand = nullptr;
   LPM_CUDA(h, cudaMallocAsync((void**)&cand, sizeof(int) * (size_t)std::max<int64_t>(hp[(size_t)n], 1), h->stream));
-  k_fill_candidates<<<grid_for(n, T), T, 0, h->stream>>>(n, d.bptr, d.lptr, d.bp2, cand_ptr, cand, cnt);
+  k_fill_candidates<<<grid_for(n, kCandWarps), 32 * kCandWarps, 0, h->stream>>>(n, d.bptr, d.lptr, d.bp2, d.blayer,
+                                                                                cand_ptr, cand, cnt);
   LPM_LAUNCHED(h, "k_fill_candidates");
+  if (*std::max_element(hc.begin(), hc.end()) > kWarpCand) {
+    k_fill_candidates_long<<<grid_for(n, T), T, 0, h->stream>>>(n, d.bptr, d.lptr, d.bp2, cand_ptr, cand, cnt);
+    LPM_LAUNCHED(h, "k_fill_candidates_long");
+  }
   LPM_CUDA(h, cudaMemcpyAsync(hc.data(), cnt, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, h->stream));
   LPM_CUDA(h, cudaStreamSynchronize(h->stream));
   std::vector<int64_t> cp((size_t)n + 1, 0);
