@@ -273,15 +273,30 @@ struct MfSlot {
   T n[3], c1, tp;
 };
 
+// Loads of data that is read once in a pass: not kept in the L1, which the
+// partners' values need (each is read by some eighteen particles).
+__device__ __forceinline__ float4 stream_load(const float4* p) {
+  float4 a;
+  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
+      : "l"(p));
+  return a;
+}
+__device__ __forceinline__ float stream_load(const float* p) {
+  float a;
+  asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(a) : "l"(p));
+  return a;
+}
+
 template <typename T, int DIM>
 __device__ __forceinline__ void mf_slot(const MfView<T>& v, int64_t slot, MfSlot<T, DIM>& o) {
   if constexpr (sizeof(T) == 4) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(v.m) + slot);
+    const float4 a = stream_load(reinterpret_cast<const float4*>(v.m) + slot);
     o.n[0] = a.x;
     o.n[1] = a.y;
     o.n[2] = DIM == 3 ? a.z : 0.f;
     o.tp = a.w;
-    o.c1 = v.m[4 * v.ns + slot];
+    o.c1 = stream_load(v.m + 4 * v.ns + slot);
   } else {
 #pragma unroll
     for (int c = 0; c < 3; ++c) o.n[c] = c < DIM ? v.m[c * v.ns + slot] : T(0);
@@ -368,6 +383,12 @@ __global__ void __launch_bounds__(256) k_mf_pass1(MfView<T> v, const T* __restri
 //           in the last block (as k_mx_residual).
 // Pipelined as pass 1; U and V of the partner are read only for the slots
 // flagged by kUVBit (a bond of the partner is damaged or broken on one side).
+// The blocks take the particles from the last: their slots are what the first
+// pass left in L2.  With that order and the slots kept out of the L1 an
+// iteration of the mixed solve takes 102 us at 61^3 particles and 343 at 101^3
+// (116 and 348 without; the order alone 108 and 336, the loads alone 103 and
+// 344).  Neither DRAM (2.4 TB/s) nor L2 binds it: the passes wait for the
+// partners' values.
 template <typename T, int DIM, int MODE, bool MASK>
 __global__ void __launch_bounds__(256) k_mf_pass2(MfView<T> v, const T* __restrict__ p, const float* __restrict__ xa,
                                                   const float* __restrict__ xb, T* __restrict__ q,
@@ -377,7 +398,7 @@ __global__ void __launch_bounds__(256) k_mf_pass2(MfView<T> v, const T* __restri
   double acc = 0.0;
   float ps = 0.f, pcs = 0.f;
   const double nd = v.norms[2];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < v.n; i += gridDim.x * blockDim.x) {
+  for (int i = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x; i < v.n; i += gridDim.x * blockDim.x) {
     T pi[3];
     mf_load<T, DIM, MODE, MASK>(v, p, xa, xb, i, pi);
     T ys[3] = {T(0), T(0), T(0)}, yc[3] = {T(0), T(0), T(0)};
