@@ -335,41 +335,97 @@ __device__ __forceinline__ void off_block(const AsmView& v, int i, int j, double
 }
 
 // A block per slice of A = K^T: lane t owns row j = 32*slice + t, the warps
-// share the row's blocks, four (a group) at a time.  Each computes K_ij with
-// i the k-th entry of conns(j) and stores its transpose in the row's k-th
-// slot: on a lattice the lanes' k-th blocks see the same neighbourhood, so
-// they walk and multiply together.
+// share the row's blocks.  Each block K_ij is computed by its row's lane and
+// its transpose stored in the row's slot.
 //
 // Bound by the FP64 pipe (13 operations per common neighbour and layer, 36 per
-// direct bond: 0.6 ms of 51^3 particles) and, next, by the L1's accesses: a
-// lane's list and records lie apart from its neighbour's.  The records bring
-// a bond's data in two loads instead of seven (sorted place, bond, its
-// opposite, four arrays).  With one warp per slice and the raw arrays it was
-// latency: 0.33 ms for any plate up to 7k rows (now 0.08 with the conditions), 1.2
-// for a 21^3 cube (0.26), 2.9 for 51^3 (1.6), 17.8 for 101^3 (8.9).
+// direct bond: 0.6 ms of 51^3 particles), if the lanes' blocks see the same
+// neighbourhood and so walk and multiply together.  On a lattice those are the
+// blocks of equal i - j, not the k-th of each row: the first row past an edge
+// of the lattice shifts them.  So the warps go through the offsets i - j of the
+// slice's longest row (`off`, in shared memory), each lane taking the block of
+// its own row at that offset if it has one, and then through the blocks at
+// other offsets.  (Where a sample of the rows' offsets has fewer than half
+// among the longest row's, the rows are taken as they are: a polycrystal of 27k
+// particles 0.49 ms, by offsets 0.54.)  The records bring a bond's data in two loads instead of
+// seven (sorted place, bond, its opposite, four arrays).
+//
+// Assembly and conditions, with one warp per slice taking the k-th blocks from
+// the raw arrays, then with the warps and the records, then by offsets: a 7k
+// plate 333, 82 and 67 us, a 21^3 cube 1203, 258 and 180 us, 51^3 2914, 1559
+// and 1080 us, 101^3 17.8, 8.9 and 7.3 ms.
 template <int DIM, bool REC>
-__global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmView v) {
+__device__ __forceinline__ void store_block(const AsmView& v, int64_t slot, int i, int j) {
+  double K[3][3];
+  if (i == j)
+    diag_block<DIM>(v, i, K);
+  else
+    off_block<DIM, REC>(v, i, j, K);
+#pragma unroll
+  for (int r = 0; r < DIM; ++r)
+#pragma unroll
+    for (int s = 0; s < DIM; ++s) v.A[(r * DIM + s) * v.nslots + slot] = K[s][r];
+}
+template <int DIM, bool REC>
+__global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmView v, int noff) {
+  extern __shared__ int off[];  // [noff], ascending
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int j = blockIdx.x * kSlice + lane;
-  if (j >= v.n) return;
-  const int len = v.rowlen[j];
-  const SellRow row = sell_row(v.sell_ptr, j);
-#pragma unroll 1
-  for (int g = warp * kVec; g < len; g += nw * kVec)
-#pragma unroll 1
-    for (int k = g; k < min(len, g + kVec); ++k) {
-      const int64_t slot = sell_slot(row, k);
-      const int i = v.scol[slot];
-      double K[3][3];
-      if (i == j)
-        diag_block<DIM>(v, i, K);
+  const int len = j < v.n ? v.rowlen[j] : 0;
+  const SellRow row = sell_row(v.sell_ptr, min(j, v.n - 1));
+  int longest = len;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+  const int src = __ffs(__ballot_sync(0xffffffffu, len == longest)) - 1;
+  int m = min(longest, noff);  // offsets
+  {
+    const int js = blockIdx.x * kSlice + src;
+    const SellRow rs = sell_row(v.sell_ptr, js);
+    for (int k = threadIdx.x; k < m; k += blockDim.x) off[k] = v.scol[sell_slot(rs, k)] - js;
+  }
+  __syncthreads();
+  auto place = [&](int o) {  // of the first offset not below o
+    int lo = 0, hi = m;
+    while (lo < hi) {
+      const int t = (lo + hi) / 2;
+      if (off[t] < o)
+        lo = t + 1;
       else
-        off_block<DIM, REC>(v, i, j, K);
-#pragma unroll
-      for (int r = 0; r < DIM; ++r)
-#pragma unroll
-        for (int s = 0; s < DIM; ++s) v.A[(r * DIM + s) * v.nslots + slot] = K[s][r];
+        hi = t;
     }
+    return lo;
+  };
+  auto listed = [&](int o) {
+    const int t = place(o);
+    return t < m && off[t] == o;
+  };
+  int found = 0, asked = 0;
+#pragma unroll 1
+  for (int q = 1; q < 4; ++q) {
+    const bool has = len > 0, in = has && listed(v.scol[sell_slot(row, len * q / 4)] - j);
+    asked += __popc(__ballot_sync(0xffffffffu, has));
+    found += __popc(__ballot_sync(0xffffffffu, in));
+  }
+  if (2 * found < asked) m = 0;
+#pragma unroll 1
+  for (int t = warp; t < m; t += nw) {
+    const int i = j + off[t];
+    int lo = 0, hi = len;  // the first block of a column not below i
+    while (lo < hi) {
+      const int k = (lo + hi) / 2;
+      if (v.scol[sell_slot(row, k)] < i)
+        lo = k + 1;
+      else
+        hi = k;
+    }
+    if (lo < len && v.scol[sell_slot(row, lo)] == i) store_block<DIM, REC>(v, sell_slot(row, lo), i, j);
+  }
+#pragma unroll 1
+  for (int k = warp; k < len; k += nw) {
+    const int64_t slot = sell_slot(row, k);
+    const int i = v.scol[slot];
+    if (!listed(i - j)) store_block<DIM, REC>(v, slot, i, j);
+  }
 }
 
 // |diag(K)|_2 (stiffness.h:269-270) and the DOFs to eliminate
@@ -593,10 +649,12 @@ int launch_assemble(lpm_handle* h, int tangent, int bc) {
   const int G = grid_for((long long)h->nslice * 32, T, 152 * 64);
   {
     const int TA = 32 * std::min(kAsmThreads / 32, std::max(1, (h->maxw + kVec - 1) / kVec));
+    const int noff = std::min(h->maxw, 48 * 1024 / (int)sizeof(int));
+    const size_t sm = sizeof(int) * (size_t)noff;
     if (dim == 3)
-      (ra ? k_assemble<3, true> : k_assemble<3, false>)<<<h->nslice, TA, 0, h->stream>>>(v);
+      (ra ? k_assemble<3, true> : k_assemble<3, false>)<<<h->nslice, TA, sm, h->stream>>>(v, noff);
     else
-      (ra ? k_assemble<2, true> : k_assemble<2, false>)<<<h->nslice, TA, 0, h->stream>>>(v);
+      (ra ? k_assemble<2, true> : k_assemble<2, false>)<<<h->nslice, TA, sm, h->stream>>>(v, noff);
     LPM_LAUNCHED(h, "k_assemble");
   }
   if (bc == LPM_BC_ELIMINATE) {
