@@ -454,38 +454,31 @@ __global__ void k_diag_norm_fixed(int n, const int* __restrict__ diag_slot, cons
 
 // Zero the rows and columns of fixed DOFs, norm on their diagonal
 // (stiffness.h:273-291).  Entry (r, s) of block (j, i) of A is K(i s, j r).
+// A block per slice, its warps sharing the rows' blocks (a warp per slice took
+// 58 us of a 21^3 cube and 77 of 51^3, here 12 and 43).
 template <int DIM>
-__global__ void __launch_bounds__(256) k_apply_bc(int n, int nslice, const int64_t* __restrict__ sell_ptr,
+__global__ void __launch_bounds__(256) k_apply_bc(int n, const int64_t* __restrict__ sell_ptr,
                                                   const int* __restrict__ scol, const int* __restrict__ rowlen,
                                                   const unsigned char* __restrict__ fixed, const double* norms,
                                                   double* __restrict__ A, int64_t nslots) {
-  const int lane = threadIdx.x & 31;
-  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int j = blockIdx.x * kSlice + lane;
+  if (j >= n) return;
   const double nd = norms[2];
-  for (long long sl = w0; sl < nslice; sl += nw) {
-    const int j = (int)(sl * kSlice) + lane;
-    if (j >= n) continue;
-    unsigned char fj[DIM];
+  unsigned char fj[DIM];
 #pragma unroll
-    for (int r = 0; r < DIM; ++r) fj[r] = fixed[DIM * j + r];
-    const int len = rowlen[j];
-    const SellRow row = sell_row(sell_ptr, j);
-    for (int k = 0; k < len; ++k) {
-      const int64_t slot = sell_slot(row, k);
-      const int i = scol[slot];
+  for (int r = 0; r < DIM; ++r) fj[r] = fixed[DIM * j + r];
+  const int len = rowlen[j];
+  const SellRow row = sell_row(sell_ptr, j);
+  for (int k = warp; k < len; k += nw) {
+    const int64_t slot = sell_slot(row, k);
+    const int i = scol[slot];
 #pragma unroll
-      for (int r = 0; r < DIM; ++r)
+    for (int r = 0; r < DIM; ++r)
 #pragma unroll
-        for (int s = 0; s < DIM; ++s)
-          if (fj[r] || fixed[DIM * i + s]) A[(r * DIM + s) * nslots + slot] = (i == j && r == s) ? nd : 0.0;
-    }
+      for (int s = 0; s < DIM; ++s)
+        if (fj[r] || fixed[DIM * i + s]) A[(r * DIM + s) * nslots + slot] = (i == j && r == s) ? nd : 0.0;
   }
-}
-
-__global__ void k_to_fp32(int64_t m, const double* __restrict__ a, float* __restrict__ b) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x)
-    b[t] = (float)a[t];
 }
 
 // 16-bit column offsets (column - row) of the slots the product reads for
@@ -507,23 +500,57 @@ __global__ void k_col_offsets(int n, const int64_t* __restrict__ sell_ptr, const
   if (bad) atomicOr(flag, 1);
 }
 
-// S_i = sum_j A_ij over the blocks of row i, summed in FP64 and rounded once.
+// The FP32 copy of the rows' slots and S_i = sum_j A_ij over row i's blocks,
+// summed in FP64 and rounded once; padding slots are zero in both.  A block
+// per slice, its warps sharing the groups, their sums added in the warps'
+// order.  Bound by the FP64 pipe where the chip is full (an addition and a
+// conversion an element: 281 us of 51^3 particles as two passes, 287 as one)
+// and by latency where it is not: 99 us of 21^3 and 21 of a 61x121 plate with
+// a thread per row, here 29 and 10.
+constexpr int kConvertWarps = 8;
 template <int DIM>
-__global__ void k_block_rowsum(int n, const int64_t* __restrict__ sell_ptr, const int* __restrict__ rowlen,
-                               const double* __restrict__ A, int64_t nslots, float* __restrict__ S) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const SellRow row = sell_row(sell_ptr, i);
-  double acc[DIM * DIM];
+__global__ void __launch_bounds__(32 * kConvertWarps) k_convert(int n, const int64_t* __restrict__ sell_ptr,
+                                                                const double* __restrict__ A, int64_t nslots,
+                                                                float* __restrict__ B, float* __restrict__ S) {
+  constexpr int E = DIM * DIM;
+  __shared__ double sum[kConvertWarps][E][32];
+  const int sl = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t base = sell_ptr[sl];
+  const int w = (int)((sell_ptr[sl + 1] - base) / kSlice), g4 = w / kVec * kVec;
+  double acc[E];
 #pragma unroll
-  for (int e = 0; e < DIM * DIM; ++e) acc[e] = 0.0;
-  for (int k = 0; k < rowlen[i]; ++k) {
-    const int64_t s = sell_slot(row, k);
+  for (int e = 0; e < E; ++e) acc[e] = 0.0;
+#pragma unroll 1
+  for (int g = warp * kVec; g < g4; g += kConvertWarps * kVec) {
+    const int64_t s = base + (int64_t)g * kSlice + lane * kVec;
 #pragma unroll
-    for (int e = 0; e < DIM * DIM; ++e) acc[e] += A[e * nslots + s];
+    for (int e = 0; e < E; ++e) {
+      const double2* q = reinterpret_cast<const double2*>(A + e * nslots + s);
+      const double2 lo = __ldcs(q), hi = __ldcs(q + 1);
+      *reinterpret_cast<float4*>(B + e * nslots + s) = make_float4((float)lo.x, (float)lo.y, (float)hi.x, (float)hi.y);
+      acc[e] += (lo.x + lo.y) + (hi.x + hi.y);
+    }
+  }
+  for (int k = g4 + warp; k < w; k += kConvertWarps) {
+    const int64_t s = base + (int64_t)k * kSlice + lane;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const double a = A[e * nslots + s];
+      B[e * nslots + s] = (float)a;
+      acc[e] += a;
+    }
   }
 #pragma unroll
-  for (int e = 0; e < DIM * DIM; ++e) S[(int64_t)i * DIM * DIM + e] = (float)acc[e];
+  for (int e = 0; e < E; ++e) sum[warp][e][lane] = acc[e];
+  __syncthreads();
+  const int i = sl * kSlice + lane;
+  if (i < n)
+    for (int e = warp; e < E; e += kConvertWarps) {
+      double t = sum[0][e][lane];
+#pragma unroll
+      for (int q = 1; q < kConvertWarps; ++q) t += sum[q][e][lane];
+      S[(int64_t)i * E + e] = (float)t;
+    }
 }
 
 }  // namespace
@@ -645,8 +672,6 @@ int launch_assemble(lpm_handle* h, int tangent, int bc) {
   AsmView v{d.bptr, d.lptr, d.sell_ptr, d.scol, d.rowlen, d.sbond, d.sp2, d.opp, d.cs, d.cs_sum, d.tsum, d.msum,
             d.Kn, d.Tv, d.bdamage, (const double2*)d.brec, d.sopp, d.A64, h->nslots, h->n, h->nslice,
             tangent == LPM_TANGENT_SYMMETRIC ? 1 : 0};
-  const int T = 256;
-  const int G = grid_for((long long)h->nslice * 32, T, 152 * 64);
   {
     const int TA = 32 * std::min(kAsmThreads / 32, std::max(1, (h->maxw + kVec - 1) / kVec));
     const int noff = std::min(h->maxw, 48 * 1024 / (int)sizeof(int));
@@ -667,10 +692,10 @@ int launch_assemble(lpm_handle* h, int tangent, int bc) {
                                                               d.fixed, d.red.partials, d.red.ticket + 1, d.norms);
     LPM_LAUNCHED(h, "k_diag_norm_fixed");
     if (dim == 3)
-      k_apply_bc<3><<<G, T, 0, h->stream>>>(h->n, h->nslice, d.sell_ptr, d.scol, d.rowlen, d.fixed, d.norms, d.A64,
+      k_apply_bc<3><<<h->nslice, 256, 0, h->stream>>>(h->n, d.sell_ptr, d.scol, d.rowlen, d.fixed, d.norms, d.A64,
                                             h->nslots);
     else
-      k_apply_bc<2><<<G, T, 0, h->stream>>>(h->n, h->nslice, d.sell_ptr, d.scol, d.rowlen, d.fixed, d.norms, d.A64,
+      k_apply_bc<2><<<h->nslice, 256, 0, h->stream>>>(h->n, d.sell_ptr, d.scol, d.rowlen, d.fixed, d.norms, d.A64,
                                             h->nslots);
     LPM_LAUNCHED(h, "k_apply_bc");
   }
@@ -709,13 +734,11 @@ int convert_A32(lpm_handle* h) {
     LPM_CUDA(h, cudaStreamSynchronize(h->stream));
     h->soff16_ok = bad == 0;
   }
-  k_to_fp32<<<grid_for((long long)vals, 256, 152 * 32), 256, 0, h->stream>>>((int64_t)vals, d.A64, d.A32);
-  LPM_LAUNCHED(h, "k_to_fp32");
   if (dim == 3)
-    k_block_rowsum<3><<<(h->n + 127) / 128, 128, 0, h->stream>>>(h->n, d.sell_ptr, d.rowlen, d.A64, h->nslots, d.S32);
+    k_convert<3><<<h->nslice, 32 * kConvertWarps, 0, h->stream>>>(h->n, d.sell_ptr, d.A64, h->nslots, d.A32, d.S32);
   else
-    k_block_rowsum<2><<<(h->n + 127) / 128, 128, 0, h->stream>>>(h->n, d.sell_ptr, d.rowlen, d.A64, h->nslots, d.S32);
-  LPM_LAUNCHED(h, "k_block_rowsum");
+    k_convert<2><<<h->nslice, 32 * kConvertWarps, 0, h->stream>>>(h->n, d.sell_ptr, d.A64, h->nslots, d.A32, d.S32);
+  LPM_LAUNCHED(h, "k_convert");
   h->a32_valid = true;
   return LPM_OK;
 }
