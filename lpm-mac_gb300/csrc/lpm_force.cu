@@ -1,9 +1,12 @@
 // Force path: bond geometry and nonlocal dilatation sums, bond forces,
 // particle forces / stress / damage_visual, residual and boundary conditions.
 //
-// One thread owns one particle and walks its bonds in stored order, so every
-// per-particle sum adds its terms in the order Particle::bond_layers lists
-// them (particle.h:163-181, 197-240).
+// One, two or four lanes of a warp own a particle (launch_geometry_force) and
+// take its bonds in stored order in turn (Particle::bond_layers,
+// particle.h:163-181, 197-240); a bond's own values are the same with any
+// number of lanes, a particle's sums are the lanes' added in a fixed order.
+#include <climits>
+
 #include "lpm_device.cuh"
 
 namespace lpm {
@@ -12,7 +15,18 @@ namespace {
 // Bond geometry + per-layer sums (bond.h:30-39, particle.h:163-181), then
 // the elastic bond force (particle_elastic.h:38-50), which needs the owner's
 // complete dLe_total: bforce = (2 Kn dLe + 2 Tv dLe_total[layer]) (1 - bdamage).
-__global__ void k_geometry_force(int n, const double* __restrict__ x, const int64_t* __restrict__ bptr,
+// Sum over the L lanes of a particle, in each of them.  (A particle's lanes
+// are neighbours in a warp and leave a kernel together.)
+template <int L>
+__device__ __forceinline__ double lanes_sum(double v) {
+  const unsigned mask = ((1u << L) - 1u) << ((threadIdx.x & 31) / L * L);
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+  return v;
+}
+
+template <int L>
+__global__ void __launch_bounds__(128) k_geometry_force(int n, const double* __restrict__ x, const int64_t* __restrict__ bptr,
                                  const int* __restrict__ bp2, const int* __restrict__ blayer,
                                  const double* __restrict__ dis0, const double* __restrict__ dLp,
                                  double* __restrict__ bdamage, const double* __restrict__ Kn,
@@ -21,13 +35,13 @@ __global__ void k_geometry_force(int n, const double* __restrict__ x, const int6
                                  double* __restrict__ dle_tot, double* __restrict__ tdle_tot,
                                  double* __restrict__ cs_sum, const double* __restrict__ damage, int damage_law,
                                  double* __restrict__ tsum, double* __restrict__ msum) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L), sub = threadIdx.x % L;
   if (i >= n) return;
   const double xi0 = x[3 * i], xi1 = x[3 * i + 1], xi2 = x[3 * i + 2];
   double dlt[NL] = {0.0, 0.0}, tdlt[NL] = {0.0, 0.0};
   double css[NL][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
   const int64_t b0 = bptr[i], b1 = bptr[i + 1];
-  for (int64_t b = b0; b < b1; ++b) {
+  for (int64_t b = b0 + sub; b < b1; b += L) {
     const int j = bp2[b];
     const double dx = xi0 - x[3 * j], dy = xi1 - x[3 * j + 1], dz = xi2 - x[3 * j + 2];
     const double d = bond_length(dx, dy, dz);
@@ -64,6 +78,11 @@ __global__ void k_geometry_force(int n, const double* __restrict__ x, const int6
   }
 #pragma unroll
   for (int l = 0; l < NL; ++l) {
+    dlt[l] = lanes_sum<L>(dlt[l]);
+    tdlt[l] = lanes_sum<L>(tdlt[l]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) css[l][k] = lanes_sum<L>(css[l][k]);
+    if (sub) continue;
     dle_tot[NL * i + l] = dlt[l];
     tdle_tot[NL * i + l] = tdlt[l];
     cs_sum[(NL * i + l) * 3 + 0] = css[l][0];
@@ -77,7 +96,7 @@ __global__ void k_geometry_force(int n, const double* __restrict__ x, const int6
   // the tangent's per-particle sums use the final bond damage (the tangent
   // is assembled after this pass): T = sum w Tv n, M = sum w (2 Kn + Tv) n n^T
   double T[2 * 3] = {0, 0, 0, 0, 0, 0}, M[2 * 6] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int64_t b = b0; b < b1; ++b) {
+  for (int64_t b = b0 + sub; b < b1; b += L) {
     const bool l1 = blayer[b] != 0;
     double f = 2. * Kn[b] * dLe[b] + 2. * Tv[b] * (l1 ? dlt[1] : dlt[0]);
     double bd = bdamage[b];
@@ -105,6 +124,11 @@ __global__ void k_geometry_force(int n, const double* __restrict__ x, const int6
     }
   }
 #pragma unroll
+  for (int k = 0; k < 6; ++k) T[k] = lanes_sum<L>(T[k]);
+#pragma unroll
+  for (int k = 0; k < 12; ++k) M[k] = lanes_sum<L>(M[k]);
+  if (sub) return;
+#pragma unroll
   for (int k = 0; k < 6; ++k) tsum[NL * 3 * i + k] = T[k];
 #pragma unroll
   for (int k = 0; k < 12; ++k) msum[NL * 6 * i + k] = M[k];
@@ -112,17 +136,18 @@ __global__ void k_geometry_force(int n, const double* __restrict__ x, const int6
 
 // Pin = sum cs * (f + f_opposite)/2 (particle.h:197-215); stress from the
 // averaged bond force (particle.h:217-240); damage_visual (particle.h:151-161).
-__global__ void k_particle_force(int n, const int64_t* __restrict__ bptr, const int* __restrict__ opp,
+template <int L>
+__global__ void __launch_bounds__(128) k_particle_force(int n, const int64_t* __restrict__ bptr, const int* __restrict__ opp,
                                  const double* __restrict__ bforce, const double* __restrict__ cs,
                                  const double* __restrict__ dis, const double* __restrict__ bdamage,
                                  const int* __restrict__ nbonds, double pvol, int nneighbors, double* __restrict__ pin,
                                  double* __restrict__ stress, double* __restrict__ dvis) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L), sub = threadIdx.x % L;
   if (i >= n) return;
   double P0 = 0, P1 = 0, P2 = 0, s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0, s5 = 0, dv = 0;
   const double Vm = pvol * nbonds[i] / nneighbors;
   const double hv = 0.5 / Vm;
-  for (int64_t b = bptr[i]; b < bptr[i + 1]; ++b) {
+  for (int64_t b = bptr[i] + sub; b < bptr[i + 1]; b += L) {
     const double f = 0.5 * (bforce[b] + bforce[opp[b]]);
     const double c0 = cs[3 * b], c1 = cs[3 * b + 1], c2 = cs[3 * b + 2];
     P0 += c0 * f;
@@ -137,6 +162,8 @@ __global__ void k_particle_force(int n, const int64_t* __restrict__ bptr, const 
     s5 += sf * c0 * c1;
     dv += bdamage[b];
   }
+  for (double* v : {&P0, &P1, &P2, &s0, &s1, &s2, &s3, &s4, &s5, &dv}) *v = lanes_sum<L>(*v);
+  if (sub) return;
   pin[3 * i] = P0;
   pin[3 * i + 1] = P1;
   pin[3 * i + 2] = P2;
@@ -317,15 +344,24 @@ int launch_geometry_force(lpm_handle* h) {
     if (st) return st;
   }
   const Dev& d = h->d;
-  const int T = 128;
-  k_geometry_force<<<grid_for(h->n, T), T, 0, h->stream>>>(h->n, d.x, d.bptr, d.bp2, d.blayer, d.dis0, d.dLp,
-                                                           d.bdamage, d.Kn, d.Tv, d.dis, d.bstrain, d.dLe, d.cs,
-                                                           d.bforce, d.dle_tot, d.tdle_tot, d.cs_sum, d.damage,
-                                                           (h->law >= 1 && h->law <= 3) ? 1 : 0, d.tsum, d.msum);
+  // Lanes of a particle.  Where the chip is full the pass is bound by the FP64
+  // pipe (some 140 operations a bond, of which the square root and the two
+  // quotients are half), and lanes only add their sums; where it is not, by a
+  // thread's chain of bonds.  us with 1, 2, 4 and 8 lanes: 1,661 particles of a
+  // plate 85, 52, 36, 37; 7,321 87, 54, 50, 78; 28,126 127, 109, 113, 225; cubes
+  // of 21^3 120, 67, 69, 87, of 51^3 637, 581, 709, 974, of 101^3 4,165, 4,226,
+  // 5,210, 7,379.  So four up to 200 threads on each of the 152 SMs, two up to
+  // all they hold.
+  const int L = h->n <= 7600 ? 4 : h->n <= 155000 ? 2 : 1;
+  const int T = 128, G = grid_for((long long)h->n * L, T, INT_MAX);
+  const auto geometry = L == 4 ? k_geometry_force<4> : L == 2 ? k_geometry_force<2> : k_geometry_force<1>;
+  const auto particle = L == 4 ? k_particle_force<4> : L == 2 ? k_particle_force<2> : k_particle_force<1>;
+  geometry<<<G, T, 0, h->stream>>>(h->n, d.x, d.bptr, d.bp2, d.blayer, d.dis0, d.dLp, d.bdamage, d.Kn, d.Tv, d.dis,
+                                   d.bstrain, d.dLe, d.cs, d.bforce, d.dle_tot, d.tdle_tot, d.cs_sum, d.damage,
+                                   (h->law >= 1 && h->law <= 3) ? 1 : 0, d.tsum, d.msum);
   LPM_LAUNCHED(h, "k_geometry_force");
-  k_particle_force<<<grid_for(h->n, T), T, 0, h->stream>>>(h->n, d.bptr, d.opp, d.bforce, d.cs, d.dis, d.bdamage,
-                                                           d.nbonds, h->particle_volume, h->nneighbors, d.pin,
-                                                           d.stress, d.dvis);
+  particle<<<G, T, 0, h->stream>>>(h->n, d.bptr, d.opp, d.bforce, d.cs, d.dis, d.bdamage, d.nbonds,
+                                   h->particle_volume, h->nneighbors, d.pin, d.stress, d.dvis);
   LPM_LAUNCHED(h, "k_particle_force");
   return LPM_OK;
 }

@@ -77,18 +77,22 @@ __global__ void k_mf_slots(int n, const int64_t* __restrict__ bptr, const int* _
 __global__ void k_mf_prep(int n, const int64_t* __restrict__ bptr, const int64_t* __restrict__ mbase,
                           const int* __restrict__ blayer, const int* __restrict__ opp, const double* __restrict__ cs,
                           const double* __restrict__ bdamage, const double* __restrict__ Kn,
-                          const double* __restrict__ Tv, const double* __restrict__ cs_sum,
-                          const double* __restrict__ tsum, int64_t ns, double* __restrict__ m64,
+                          const double* __restrict__ Tv, const double* __restrict__ cs_sum, int64_t ns,
+                          double* __restrict__ m64,
                           float* __restrict__ m32, double* __restrict__ S64, double* __restrict__ U64,
                           double* __restrict__ V64, float* __restrict__ S32, float* __restrict__ U32,
                           float* __restrict__ V32) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t s0 = mbase[i / 32] + (i % 32);
+  // sums of the opposite bonds' n' and t' n', and of the bonds' own in the same
+  // order: for intact bonds the two cancel exactly
   double so[NL][3] = {{0, 0, 0}, {0, 0, 0}}, to[NL][3] = {{0, 0, 0}, {0, 0, 0}};
+  double sn[NL][3] = {{0, 0, 0}, {0, 0, 0}}, tn[NL][3] = {{0, 0, 0}, {0, 0, 0}};
   int k = 0;
   for (int64_t b = bptr[i]; b < bptr[i + 1]; ++b, ++k) {
     const int bo = opp[b];
+    const double to1 = (1.0 - bdamage[b]) * Tv[b];
     const double w = 1.0 - bdamage[bo], tv = Tv[bo];
     const double tp = w * tv, c1 = w * (2.0 * Kn[bo] + tv) - tp;
     const double v[kMfFields] = {cs[3 * (int64_t)bo], cs[3 * (int64_t)bo + 1], cs[3 * (int64_t)bo + 2], c1, tp};
@@ -103,6 +107,8 @@ __global__ void k_mf_prep(int n, const int64_t* __restrict__ bptr, const int64_t
     for (int c = 0; c < 3; ++c) {
       so[l][c] += v[c];
       to[l][c] += tp * v[c];
+      sn[l][c] += cs[3 * b + c];
+      tn[l][c] += to1 * cs[3 * b + c];
     }
   }
 #pragma unroll
@@ -110,7 +116,7 @@ __global__ void k_mf_prep(int n, const int64_t* __restrict__ bptr, const int64_t
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int64_t q = ((int64_t)i * NL + l) * 3 + c;
-      const double S = cs_sum[q], U = S + so[l][c], V = tsum[q] + to[l][c];
+      const double S = cs_sum[q], U = sn[l][c] + so[l][c], V = tn[l][c] + to[l][c];
       S64[q] = S;
       U64[q] = U;
       V64[q] = V;
@@ -693,7 +699,7 @@ int mf_assemble(lpm_handle* h, int tangent, int bc) {
   }
   const int n = h->n;
   k_mf_prep<<<grid_for(n, 128), 128, 0, h->stream>>>(n, d.bptr, d.mbase, d.blayer, d.opp, d.cs, d.bdamage, d.Kn,
-                                                      d.Tv, d.cs_sum, d.tsum, h->mslots, d.m64, d.m32, d.mS64, d.mU64,
+                                                      d.Tv, d.cs_sum, h->mslots, d.m64, d.m32, d.mS64, d.mU64,
                                                       d.mV64, d.mS32, d.mU32, d.mV32);
   LPM_LAUNCHED(h, "k_mf_prep");
   k_mf_flags<<<grid_for(n, 128), 128, 0, h->stream>>>(n, d.mbase, d.mU64, d.mV64, d.mp2);
