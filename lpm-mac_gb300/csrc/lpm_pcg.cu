@@ -27,7 +27,7 @@
 //
 // Measured on GB300, us per iteration of the mixed solve, here against the
 // better of the graph and the persistent loop of lpm_cg.cu: hexagonal plates
-// of 1,661 rows 7.5 (16.1), 28,126 rows 8.5 (18.2), 80,401 rows 12.8 (21.9)
+// of 1,661 rows 6.7 (16.1), 28,126 rows 7.8 (18.2), 80,401 rows 12.6 (21.9)
 // and 112,658 rows 15.9 (24.7); simple cubes of 21^3 9.9 (25.5), 31^3 17 (30)
 // and 41^3 41 (50); a BCC polycrystal of 27,287 rows 12.8 (27).  Of an
 // iteration of the 28k plate (16.5k cycles) the product takes 4.0k, the two
@@ -345,7 +345,7 @@ __device__ __forceinline__ void warp_to_shared(PcgShared& sh, int ls, double (&v
 // the e a block's rows need travel while block 0 forms beta.  Bound by those
 // trips through L2, one after the other: us per iteration here against
 // k_mx_persistent, whose grid barriers they replace, 61x121 plate (363 coarse
-// DOFs) 21 (43), 201x401 plate 25 (43), 21^3 cube 25 (65), 41^3 cube 63 (87).
+// DOFs) 19 (43), 201x401 plate 25 (43), 21^3 cube 25 (65), 41^3 cube 63 (87).
 struct CoarseRow {
   float d[3];         // offset from the aggregate's centroid
   unsigned agg_mask;  // aggregate among the block's (low 16 bits), eliminated DOFs (bits 16..)
@@ -1346,10 +1346,14 @@ int run_mixed_dim(lpm_handle* h, bool keep) {
   Dev& d = h->d;
   PcgPlan& pl = h->pcg;
   using Fn = void (*)(PcgMixedArgs);
-  constexpr int kBound = kPcgThreads<DIM>, kWide = kPcgWideThreads<DIM>;
+  constexpr int kBound = kPcgThreads<DIM>, kWide = kPcgWideThreads<DIM>, kNarrow = kPcgNarrowThreads;
   const bool wide = (pl.S + 1) * 32 > kBound;
-  const Fn fn = wide ? (keep ? k_pcg_mixed<DIM, true, kWide, COARSE> : k_pcg_mixed<DIM, false, kWide, COARSE>)
-                     : (keep ? k_pcg_mixed<DIM, true, kBound, COARSE> : k_pcg_mixed<DIM, false, kBound, COARSE>);
+  // the narrow form, unless it has a warp for each slice where the other has two
+  const int share = (kNarrow / 32 - 1) / pl.S;
+  const bool narrow = DIM == 2 && share > 0 && (share > 1 || (kBound / 32 - 1) / pl.S == 1);
+  const Fn fn = narrow ? k_pcg_mixed<DIM, true, kNarrow, COARSE>
+                : wide ? (keep ? k_pcg_mixed<DIM, true, kWide, COARSE> : k_pcg_mixed<DIM, false, kWide, COARSE>)
+                       : (keep ? k_pcg_mixed<DIM, true, kBound, COARSE> : k_pcg_mixed<DIM, false, kBound, COARSE>);
   PcgShape& sh = COARSE ? pl.mixed_coarse : pl.mixed;
   const int cmaxrows = COARSE ? (h->cnc + pl.G - 1) / pl.G : 0;
   if (!sh.state) {
@@ -1358,7 +1362,7 @@ int run_mixed_dim(lpm_handle* h, bool keep) {
                                        sizeof(double) * (size_t)(1 + cmaxrows) * h->cnc +
                                        (sizeof(float) * kModes<DIM> + 2 * sizeof(int)) * (size_t)pl.cmaxagg
                                  : 0;
-    sh.state = shape_on_plan(h, (const void*)fn, wide ? kWide : kBound, kPcgUnit<DIM>, sizeof(float) * DIM,
+    sh.state = shape_on_plan(h, (const void*)fn, narrow ? kNarrow : wide ? kWide : kBound, kPcgUnit<DIM>, sizeof(float) * DIM,
                              sizeof(double) * DIM, sizeof(float) * (DIM * DIM + DIM), coarse, &sh)
                    ? 1
                    : -1;

@@ -11,11 +11,18 @@ constexpr int kPcgMaxSlices = 32;   // 32-row slices of a block (a lane each in 
 
 // Threads per block, one block per SM, the message warp included: registers
 // for an operator group in flight beside the one in use (2-D: 80, 3-D: 128).
-// The wide form has a warp more for 2-D blocks of 24 slices (72 registers).
+// The wide form has a warp more for 2-D blocks of 24 slices (72 registers),
+// the narrow one 128 registers in 2-D too: at 80 the message warp keeps part of
+// its records in local memory, on the path from one iteration to the next (us
+// per iteration of the mixed solve, 768 and 512 threads: plates of 3.6k rows
+// 7.7 and 6.75, 28k 8.8 and 7.9, 60k 11.6 and 10.6).  It stands back where its
+// fifteen compute warps leave a slice one and the others leave it two (45k
+// rows: 9.6 and 9.9).
 template <int DIM>
 constexpr int kPcgThreads = DIM == 3 ? 512 : 768;
 template <int DIM>
 constexpr int kPcgWideThreads = DIM == 3 ? 512 : 800;
+constexpr int kPcgNarrowThreads = 512;
 
 // Shared memory of one resident group of a slice: 32 rows x four blocks of
 // DIM*DIM FP32 values and their 16-bit positions.

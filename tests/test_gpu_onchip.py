@@ -140,3 +140,30 @@ def test_mixed_solve_on_chip_with_damage():
     if st == capi.OK:
         r, bound = _held(A, b, x)
         assert r <= bound and abs(it - itg) <= 0.05 * itg + 4
+
+
+@pytest.mark.parametrize("nx,ny", [(190, 190), (215, 215), (240, 240), (275, 275), (336, 336)])
+def test_mixed_solve_on_chip_of_many_slices_a_block(nx, ny):
+    """8, 10, 12, 16 and 24 slices in the largest block: a block's threads and
+    the warps of a slice change between them."""
+    g = make_gpu(*plate(nx, ny))
+    xyz = g.download(capi.F_XYZ)
+    mask = np.zeros((g.n, 3), np.int32)
+    mask[xyz[:, 1] < xyz[:, 1].min() + 1e-9, :2] = 1
+    mask[xyz[:, 1] > xyz[:, 1].max() - 1e-9, 1] = 1
+    g.set_mask(mask)
+    g.update()
+    g.assemble(capi.TANGENT_SYMMETRIC, capi.BC_ELIMINATE)
+    b = (np.random.default_rng(3).standard_normal((g.n, 2)) * (1 - mask[:, :2])).ravel()
+    g.upload(capi.F_RESIDUAL, b)
+    g.reset_stats()
+    it, rr, st = g.solve(capi.PREC_MIXED, TOL)
+    x = g.download(capi.F_DISP)
+    cptr, _ = g.pattern()
+    rows = np.abs(g.K_bsr()).reshape(-1, 4).sum(1)  # each block's entries, an upper bound of its share of |A|
+    norm = np.add.reduceat(rows, cptr[:-1]).max()
+    r = np.linalg.norm(b - np.ravel(g.apply_operator(x)))
+    bound = TOL * np.linalg.norm(b) + 1e-13 * norm * np.linalg.norm(x)
+    print("[on chip] plate %dx%d: %d iterations, residual %.2e of a bound of %.2e" % (nx, ny, it, r, bound))
+    assert st == capi.OK and g.stats()["persistent_solves"] == 1 and r <= bound
+    g.close()
