@@ -327,21 +327,55 @@ __device__ __forceinline__ void mf_hf(const MfView<T>& v, int j, int l, T (&o)[2
   }
 }
 
+// L lanes of a warp to a particle: lane t takes particle t % (32/L) of the
+// warp's and, of its slots, those t / (32/L) + L q, so that the lanes of one
+// slot stay beside each other.
+template <int L>
+__device__ __forceinline__ int mf_part() {
+  return (int)(threadIdx.x & 31) / (32 / L);
+}
+template <int L>
+__device__ __forceinline__ int mf_first(int block) {
+  return (int)((block * blockDim.x + (threadIdx.x & ~31u)) / L);
+}
+template <int L>
+__device__ __forceinline__ int mf_particle(int w0, int n) {  // (a lane past the last walks along with it)
+  return min(w0 + (int)(threadIdx.x & 31) % (32 / L), n - 1);
+}
+// The lanes' sums together, in each of them: pairs in FP32, plain in FP64.
+template <int L, int K, typename T>
+__device__ __forceinline__ void mf_combine(T (&s)[K], T (&c)[K]) {
+#pragma unroll
+  for (int o = 16; o >= 32 / L; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const T so = __shfl_xor_sync(0xffffffffu, s[k], o);
+      if constexpr (sizeof(T) == 4) {
+        const T co = __shfl_xor_sync(0xffffffffu, c[k], o);
+        df_add(s[k], c[k], so, co);
+      } else {
+        s[k] += so;
+      }
+    }
+}
+
 // Pass 1: H_j = sum n'.(p_m - p_j), F_j = sum t' n'.(p_m - p_j) per layer
 // over j's bonds.  FP32 sums are compensated and rounded once.  The loop is
 // software-pipelined: the next slot's coefficients and partner values, and
 // the partner word of the slot after it, are loaded while the current slot
 // is used.
-template <typename T, int DIM, int MODE, bool MASK>
+template <typename T, int DIM, int MODE, bool MASK, int L>
 __global__ void __launch_bounds__(256) k_mf_pass1(MfView<T> v, const T* __restrict__ p, const float* __restrict__ xa,
                                                   const float* __restrict__ xb, const CgScalars* cg) {
   if (cg->done || (MODE == 1 && !cg->ru)) return;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < v.n; j += gridDim.x * blockDim.x) {
+  const int part = mf_part<L>();
+  for (int w0 = mf_first<L>(blockIdx.x); w0 < v.n; w0 += gridDim.x * blockDim.x / L) {
+    const int j = mf_particle<L>(w0, v.n);
     T pj[3];
     mf_load<T, DIM, MODE, MASK>(v, p, xa, xb, j, pj);
     const int sl = j / 32;
-    const int64_t s0 = v.mbase[sl] + (j % 32);
-    const int len = (int)((v.mbase[sl + 1] - v.mbase[sl]) / 32);
+    const int64_t s0 = v.mbase[sl] + (j % 32) + 32 * part;
+    const int len = ((int)((v.mbase[sl + 1] - v.mbase[sl]) / 32) - part + L - 1) / L;  // this lane's slots
     T hs[NL] = {T(0), T(0)}, hc[NL] = {T(0), T(0)}, fs[NL] = {T(0), T(0)}, fc[NL] = {T(0), T(0)};
     MfSlot<T, DIM> cur{}, nxt{};
     T pc[3] = {T(0), T(0), T(0)}, pn[3] = {T(0), T(0), T(0)};
@@ -350,31 +384,43 @@ __global__ void __launch_bounds__(256) k_mf_pass1(MfView<T> v, const T* __restri
       wc = v.mp2[s0];
       mf_slot<T, DIM>(v, s0, cur);
       mf_load<T, DIM, MODE, MASK>(v, p, xa, xb, (int)(wc & kIdMask), pc);
-      if (len > 1) wn = v.mp2[s0 + 32];
+      if (len > 1) wn = v.mp2[s0 + 32 * L];
     }
     for (int k = 0; k < len; ++k) {
       if (k + 1 < len) {
-        mf_slot<T, DIM>(v, s0 + 32 * (int64_t)(k + 1), nxt);
+        mf_slot<T, DIM>(v, s0 + 32 * L * (int64_t)(k + 1), nxt);
         mf_load<T, DIM, MODE, MASK>(v, p, xa, xb, (int)(wn & kIdMask), pn);
-        if (k + 2 < len) w2 = v.mp2[s0 + 32 * (int64_t)(k + 2)];
+        if (k + 2 < len) w2 = v.mp2[s0 + 32 * L * (int64_t)(k + 2)];
       }
       const int l = (wc & kLayerBit) ? 1 : 0;
       T s = cur.n[0] * (pc[0] - pj[0]);
 #pragma unroll
       for (int c = 1; c < DIM; ++c) s = fma(cur.n[c], pc[c] - pj[c], s);
+      T h0 = l ? hs[1] : hs[0], h1 = l ? hc[1] : hc[0], f0 = l ? fs[1] : fs[0], f1 = l ? fc[1] : fc[0];
       if constexpr (sizeof(T) == 4) {
-        df_add(hs[l], hc[l], s, 0.f);
-        dot2_acc(fs[l], fc[l], cur.tp, s);
+        df_add(h0, h1, s, 0.f);
+        dot2_acc(f0, f1, cur.tp, s);
       } else {
-        hs[l] += s;
-        fs[l] = fma(cur.tp, s, fs[l]);
+        h0 += s;
+        f0 = fma(cur.tp, s, f0);
       }
+      hs[0] = l ? hs[0] : h0;
+      hc[0] = l ? hc[0] : h1;
+      fs[0] = l ? fs[0] : f0;
+      fc[0] = l ? fc[0] : f1;
+      hs[1] = l ? h0 : hs[1];
+      hc[1] = l ? h1 : hc[1];
+      fs[1] = l ? f0 : fs[1];
+      fc[1] = l ? f1 : fc[1];
       cur = nxt;
       wc = wn;
       wn = w2;
 #pragma unroll
       for (int c = 0; c < 3; ++c) pc[c] = pn[c];
     }
+    mf_combine<L, NL>(hs, hc);
+    mf_combine<L, NL>(fs, fc);
+    if (part || w0 + (int)(threadIdx.x & 31) >= v.n) continue;
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
       v.HF[((int64_t)l * v.n + j) * 2] = hs[l] + hc[l];
@@ -389,14 +435,16 @@ __global__ void __launch_bounds__(256) k_mf_pass1(MfView<T> v, const T* __restri
 //           in the last block (as k_mx_residual).
 // Pipelined as pass 1; U and V of the partner are read only for the slots
 // flagged by kUVBit (a bond of the partner is damaged or broken on one side).
+// The layers' sums are held by selection: indexed they lay in local memory
+// (100 us of an iteration at 61^3 particles, now 90; 333 at 101^3, now 287).
 // The blocks take the particles from the last: their slots are what the first
 // pass left in L2.  With that order and the slots kept out of the L1 an
 // iteration of the mixed solve takes 102 us at 61^3 particles and 343 at 101^3
 // (116 and 348 without; the order alone 108 and 336, the loads alone 103 and
 // 344).  Neither DRAM (2.4 TB/s) nor L2 binds it: the passes wait for the
 // partners' values.
-template <typename T, int DIM, int MODE, bool MASK>
-__global__ void __launch_bounds__(256) k_mf_pass2(MfView<T> v, const T* __restrict__ p, const float* __restrict__ xa,
+template <typename T, int DIM, int MODE, bool MASK, int L>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_mf_pass2(MfView<T> v, const T* __restrict__ p, const float* __restrict__ xa,
                                                   const float* __restrict__ xb, T* __restrict__ q,
                                                   float* __restrict__ qlo, const double* __restrict__ rhs,
                                                   CgScalars* cg, double* partials, unsigned int* ticket) {
@@ -404,23 +452,26 @@ __global__ void __launch_bounds__(256) k_mf_pass2(MfView<T> v, const T* __restri
   double acc = 0.0;
   float ps = 0.f, pcs = 0.f;
   const double nd = v.norms[2];
-  for (int i = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x; i < v.n; i += gridDim.x * blockDim.x) {
+  const int part = mf_part<L>();
+  for (int w0 = mf_first<L>(gridDim.x - 1 - blockIdx.x); w0 < v.n; w0 += gridDim.x * blockDim.x / L) {
+    const int i = mf_particle<L>(w0, v.n);
     T pi[3];
     mf_load<T, DIM, MODE, MASK>(v, p, xa, xb, i, pi);
     T ys[3] = {T(0), T(0), T(0)}, yc[3] = {T(0), T(0), T(0)};
     const T* Ri = v.R + (int64_t)i * 9;
+    if (part == 0)
 #pragma unroll
-    for (int r = 0; r < DIM; ++r)
+      for (int r = 0; r < DIM; ++r)
 #pragma unroll
-      for (int c = 0; c < DIM; ++c) {
+        for (int c = 0; c < DIM; ++c) {
         if constexpr (sizeof(T) == 4)
           dot2_acc(ys[r], yc[r], Ri[r * 3 + c], pi[c]);
         else
           ys[r] = fma(Ri[r * 3 + c], pi[c], ys[r]);
       }
     const int sl = i / 32;
-    const int64_t s0 = v.mbase[sl] + (i % 32);
-    const int len = (int)((v.mbase[sl + 1] - v.mbase[sl]) / 32);
+    const int64_t s0 = v.mbase[sl] + (i % 32) + 32 * part;
+    const int len = ((int)((v.mbase[sl + 1] - v.mbase[sl]) / 32) - part + L - 1) / L;  // this lane's slots
     T as[NL] = {T(0), T(0)}, ac[NL] = {T(0), T(0)};
     MfSlot<T, DIM> cur{}, nxt{};
     T pc[3] = {T(0), T(0), T(0)}, pn[3] = {T(0), T(0), T(0)}, hc2[2] = {T(0), T(0)}, hn2[2] = {T(0), T(0)};
@@ -431,15 +482,15 @@ __global__ void __launch_bounds__(256) k_mf_pass2(MfView<T> v, const T* __restri
       const int j0 = (int)(wc & kIdMask), l0 = (wc & kLayerBit) ? 1 : 0;
       mf_load<T, DIM, MODE, MASK>(v, p, xa, xb, j0, pc);
       mf_hf<T>(v, j0, l0, hc2);
-      if (len > 1) wn = v.mp2[s0 + 32];
+      if (len > 1) wn = v.mp2[s0 + 32 * L];
     }
     for (int k = 0; k < len; ++k) {
       if (k + 1 < len) {
-        mf_slot<T, DIM>(v, s0 + 32 * (int64_t)(k + 1), nxt);
+        mf_slot<T, DIM>(v, s0 + 32 * L * (int64_t)(k + 1), nxt);
         const int j1 = (int)(wn & kIdMask), l1 = (wn & kLayerBit) ? 1 : 0;
         mf_load<T, DIM, MODE, MASK>(v, p, xa, xb, j1, pn);
         mf_hf<T>(v, j1, l1, hn2);
-        if (k + 2 < len) w2 = v.mp2[s0 + 32 * (int64_t)(k + 2)];
+        if (k + 2 < len) w2 = v.mp2[s0 + 32 * L * (int64_t)(k + 2)];
       }
       const int j = (int)(wc & kIdMask);
       const int l = (wc & kLayerBit) ? 1 : 0;
@@ -467,10 +518,15 @@ __global__ void __launch_bounds__(256) k_mf_pass2(MfView<T> v, const T* __restri
         else
           ys[r] = fma(cur.n[r], coef, ys[r]);
       }
+      T a0 = l ? as[1] : as[0], a1 = l ? ac[1] : ac[0];
       if constexpr (sizeof(T) == 4)
-        dot2_acc(as[l], ac[l], cur.tp, s);
+        dot2_acc(a0, a1, cur.tp, s);
       else
-        as[l] = fma(cur.tp, s, as[l]);
+        a0 = fma(cur.tp, s, a0);
+      as[0] = l ? as[0] : a0;
+      ac[0] = l ? ac[0] : a1;
+      as[1] = l ? a0 : as[1];
+      ac[1] = l ? a1 : ac[1];
       cur = nxt;
       wc = wn;
       wn = w2;
@@ -479,6 +535,9 @@ __global__ void __launch_bounds__(256) k_mf_pass2(MfView<T> v, const T* __restri
       hc2[0] = hn2[0];
       hc2[1] = hn2[1];
     }
+    mf_combine<L, 3>(ys, yc);
+    mf_combine<L, NL>(as, ac);
+    if (part || w0 + (int)(threadIdx.x & 31) >= v.n) continue;
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
       const T* Si = v.S + ((int64_t)i * NL + l) * 3;
@@ -629,54 +688,75 @@ MfView<T> mf_view(lpm_handle* h) {
                      h->n};
 }
 
-// Grid of the two passes: one thread per particle, grid-stride, at most as
-// many blocks as the reduction partials hold.
-int mf_grid(const lpm_handle* h) { return grid_for(h->n, 256, kMaxRedBlocks); }
+// Lanes of a particle in the passes.  With one, 61^3 particles are 1.5 waves of
+// resident threads, and a thread's chain of slots sets the time; with two the
+// waves are shorter and more even.  Where there are many waves the second lane
+// only adds its sums, and in FP64 the passes are bound by its pipe earlier.  us
+// per iteration with one, two and four lanes: mixed solve, 21^3 particles 43.5,
+// 36.8, 33.6; 41^3 55, 47, 53; 61^3 90, 88, 103; 101^3 287, 308, 372; FP64 solve,
+// 21^3 64, 45, 37; 41^3 109, 116, 139; 61^3 288, 306, 378.
+int mf_lanes(const lpm_handle* h, bool fp32) { return h->n <= (fp32 ? 311000 : 32000) ? 2 : 1; }
 
-template <typename T, int DIM, bool MASK>
-int mf_product_dim(lpm_handle* h, cudaGraph_t g, const cudaGraphNode_t* dep, const T* p, T* q, float* qlo,
+// Grid of the two passes: grid-stride, at most as many blocks as the
+// reduction partials hold.
+int mf_grid(const lpm_handle* h, int lanes) { return grid_for((long long)h->n * lanes, 256, kMaxRedBlocks); }
+
+template <typename T, int DIM, bool MASK, int L>
+int mf_product_lanes(lpm_handle* h, cudaGraph_t g, const cudaGraphNode_t* dep, const T* p, T* q, float* qlo,
                    cudaGraphNode_t* last) {
   Dev& d = h->d;
   const MfView<T> v = mf_view<T>(h);
-  const int G = mf_grid(h);
+  const int G = mf_grid(h, L);
   const float* nf = nullptr;
   const double* nb = nullptr;
   if (!g) {
-    k_mf_pass1<T, DIM, 0, MASK><<<G, 256, 0, h->stream>>>(v, p, nf, nf, d.cg);
+    k_mf_pass1<T, DIM, 0, MASK, L><<<G, 256, 0, h->stream>>>(v, p, nf, nf, d.cg);
     LPM_LAUNCHED(h, "k_mf_pass1");
-    k_mf_pass2<T, DIM, 0, MASK><<<G, 256, 0, h->stream>>>(v, p, nf, nf, q, qlo, nb, d.cg, d.red.partials,
+    k_mf_pass2<T, DIM, 0, MASK, L><<<G, 256, 0, h->stream>>>(v, p, nf, nf, q, qlo, nb, d.cg, d.red.partials,
                                                             d.red.ticket + 3);
     LPM_LAUNCHED(h, "k_mf_pass2");
     return LPM_OK;
   }
   cudaGraphNode_t n1;
-  LPM_CUDA(h, add_kernel(&n1, g, dep, k_mf_pass1<T, DIM, 0, MASK>, G, 256, v, p, nf, nf, (const CgScalars*)d.cg));
-  LPM_CUDA(h, add_kernel(last, g, &n1, k_mf_pass2<T, DIM, 0, MASK>, G, 256, v, p, nf, nf, q, qlo, nb, d.cg,
+  LPM_CUDA(h, add_kernel(&n1, g, dep, k_mf_pass1<T, DIM, 0, MASK, L>, G, 256, v, p, nf, nf, (const CgScalars*)d.cg));
+  LPM_CUDA(h, add_kernel(last, g, &n1, k_mf_pass2<T, DIM, 0, MASK, L>, G, 256, v, p, nf, nf, q, qlo, nb, d.cg,
                          d.red.partials, d.red.ticket + 3));
   return LPM_OK;
 }
 
-template <int DIM>
-int mf_residual_dim(lpm_handle* h, cudaGraph_t g, const cudaGraphNode_t* dep, cudaGraphNode_t* last) {
+template <typename T, int DIM, bool MASK>
+int mf_product_dim(lpm_handle* h, cudaGraph_t g, const cudaGraphNode_t* dep, const T* p, T* q, float* qlo,
+                   cudaGraphNode_t* last) {
+  return mf_lanes(h, sizeof(T) == 4) == 2 ? mf_product_lanes<T, DIM, MASK, 2>(h, g, dep, p, q, qlo, last)
+                                          : mf_product_lanes<T, DIM, MASK, 1>(h, g, dep, p, q, qlo, last);
+}
+
+template <int DIM, int L>
+int mf_residual_lanes(lpm_handle* h, cudaGraph_t g, const cudaGraphNode_t* dep, cudaGraphNode_t* last) {
   Dev& d = h->d;
   const MfView<double> v = mf_view<double>(h);
-  const int G = mf_grid(h);
+  const int G = mf_grid(h, L);
   float* nf = nullptr;
   if (!g) {
-    k_mf_pass1<double, DIM, 1, false><<<G, 256, 0, h->stream>>>(v, d.x64, d.x32, d.x32lo, d.cg);
+    k_mf_pass1<double, DIM, 1, false, L><<<G, 256, 0, h->stream>>>(v, d.x64, d.x32, d.x32lo, d.cg);
     LPM_LAUNCHED(h, "k_mf_pass1");
-    k_mf_pass2<double, DIM, 1, false><<<G, 256, 0, h->stream>>>(v, d.x64, d.x32, d.x32lo, d.r64, nf, d.rhs, d.cg,
+    k_mf_pass2<double, DIM, 1, false, L><<<G, 256, 0, h->stream>>>(v, d.x64, d.x32, d.x32lo, d.r64, nf, d.rhs, d.cg,
                                                                   d.red.partials, d.red.ticket + 6);
     LPM_LAUNCHED(h, "k_mf_pass2");
     return LPM_OK;
   }
   cudaGraphNode_t n1;
-  LPM_CUDA(h, add_kernel(&n1, g, dep, k_mf_pass1<double, DIM, 1, false>, G, 256, v, (const double*)d.x64,
+  LPM_CUDA(h, add_kernel(&n1, g, dep, k_mf_pass1<double, DIM, 1, false, L>, G, 256, v, (const double*)d.x64,
                          (const float*)d.x32, (const float*)d.x32lo, (const CgScalars*)d.cg));
-  LPM_CUDA(h, add_kernel(last, g, &n1, k_mf_pass2<double, DIM, 1, false>, G, 256, v, (const double*)d.x64,
+  LPM_CUDA(h, add_kernel(last, g, &n1, k_mf_pass2<double, DIM, 1, false, L>, G, 256, v, (const double*)d.x64,
                          (const float*)d.x32, (const float*)d.x32lo, d.r64, nf, (const double*)d.rhs, d.cg,
                          d.red.partials, d.red.ticket + 6));
   return LPM_OK;
+}
+template <int DIM>
+int mf_residual_dim(lpm_handle* h, cudaGraph_t g, const cudaGraphNode_t* dep, cudaGraphNode_t* last) {
+  return mf_lanes(h, false) == 2 ? mf_residual_lanes<DIM, 2>(h, g, dep, last)
+                                 : mf_residual_lanes<DIM, 1>(h, g, dep, last);
 }
 
 template <bool MASK>
