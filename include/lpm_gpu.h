@@ -310,8 +310,11 @@ int lpm_set_kernel_timing(lpm_handle* h, int on);
  *                           with the loop and reliable-update conditions set
  *                           on the device.
  *   LPM_CG_LOOP_PERSISTENT  one cooperative kernel per solve whose blocks
- *                           stay resident and meet at grid barriers (three
- *                           per iteration, two more per reliable update);
+ *                           stay resident: with the working set in shared
+ *                           memory and two sums over the blocks per
+ *                           iteration where one wave of blocks holds the
+ *                           rows, else meeting at grid barriers (three per
+ *                           iteration, two more per reliable update);
  *                           for systems too small to fill the GPU, where the
  *                           graph's per-kernel overheads dominate.  Same
  *                           recurrence, same stopping rule; the sums are
@@ -322,8 +325,8 @@ int lpm_set_kernel_timing(lpm_handle* h, int on);
  *                           mixed solve that cannot run on chip, the FP32
  *                           operator fits in half of L2); else the graph.
  * Both precisions have both loops.  The matrix-free operator and kernel
- * timing always use the graph or host loop.  A barrier wait that gives up (a
- * bounded spin) ends the solve with LPM_ERR_STATE. */
+ * timing always use the graph or host loop.  A wait that gives up (a bounded
+ * spin) ends the solve with LPM_ERR_STATE. */
 #define LPM_CG_LOOP_AUTO 0
 #define LPM_CG_LOOP_GRAPH 1
 #define LPM_CG_LOOP_PERSISTENT 2
