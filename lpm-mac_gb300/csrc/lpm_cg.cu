@@ -429,7 +429,10 @@ __global__ void __launch_bounds__(256) k_mx_update(int64_t ndof, float* __restri
                                                    const float* __restrict__ qlo, const float* __restrict__ invd,
                                                    CgScalars* cg, double* partials, unsigned int* ticket,
                                                    cudaGraphConditionalHandle ru_cond) {
-  if (cg->done) return;
+  if (cg->done) {
+    if (ru_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(ru_cond, 0u);
+    return;
+  }
   const float ah = cg->alpha32, al = cg->alpha32lo;
   // |r|^2 and r.z as compensated double-float sums, FP64 only per warp
   float s[2] = {0.f, 0.f}, c[2] = {0.f, 0.f};
@@ -1141,6 +1144,16 @@ __global__ void __launch_bounds__(kPcg64Threads, 1) k_cg_persistent(PcgFp64 a) {
   }
 }
 
+// CG iterations in one pass of a solve graph's loop: the loop condition costs
+// some 5 us a pass, and what follows the end of a solve in its pass is launches
+// that return at once.  us per iteration with one, two, four and eight: 401x401
+// plate 46.4, 43.9, 43.2, 42.1; matrix-free 41^3 particles 46.7, 44.3, 43.1,
+// 42.1, 61^3 87.4, 85.4, 84.2, 83.3; 61^3 assembled 114.3, 112.0, 111.3, 110.4,
+// 101^3 447.0, 444.6, 443.3, 442.3; FP64 61^3 261.3, 259.3, 258.4, 257.9.
+// Against that a solve of one iteration takes 135, 143, 158 and 195 us, and the
+// first one's graph 0.04, 0.1 and 0.23 ms more than with one.
+constexpr int kGraphIterations = 4;
+
 // Grid of the FP64 row kernels (product, true residual): these are bound by
 // the FP64 pipe, and measured faster with several waves of blocks than with
 // one resident wave (0.99 against 1.06 ms per product at 101^3).
@@ -1270,7 +1283,7 @@ int run_cg(lpm_handle* h, const T* A, const T* b, T* x, T* r, T* p, T* q, const 
       LPM_CUDA(h, cudaGraphLaunch(h->fp_exec, h->stream));
       LPM_CUDA(h, cudaMemcpyAsync(h->h_cg, d.cg, sizeof(CgScalars), cudaMemcpyDeviceToHost, h->stream));
       LPM_CUDA(h, cudaStreamSynchronize(h->stream));
-      h->stats.kernel_launches += 3 * h->h_cg->graph_passes;
+      h->stats.kernel_launches += 3 * kGraphIterations * h->h_cg->graph_passes;
       return LPM_OK;
     }
   }
@@ -1463,7 +1476,8 @@ int run_persistent_mixed(lpm_handle* h, const SellView& sv, int grid, int thread
 }
 
 // The mixed solve's iteration loop as one graph:
-//   while (loop_cond) { spmv; update; if (ru_cond) { residual; replace } pupdate }
+//   while (loop_cond) { kGraphIterations times:
+//                       spmv; update; if (ru_cond) { residual; replace } pupdate }
 // update sets ru_cond (a reliable update is due) and pupdate sets
 // loop_cond (the solve goes on), so a whole solve is one graph launch with
 // no host round trip and no launch of an idle reliable-update kernel.
@@ -1478,7 +1492,7 @@ int build_mixed_graph(lpm_handle* h, const SellView& sv, const MixedGrids& mg) {
   cudaGraph_t g;
   LPM_CUDA(h, cudaGraphCreate(&g, 0));
   h->mx_graph = g;
-  cudaGraphConditionalHandle loop_cond, ru_cond;
+  cudaGraphConditionalHandle loop_cond;
   LPM_CUDA(h, cudaGraphConditionalHandleCreate(&loop_cond, g, 1u, cudaGraphCondAssignDefault));
   cudaGraphNodeParams wp = {};
   wp.type = cudaGraphNodeTypeConditional;
@@ -1488,45 +1502,51 @@ int build_mixed_graph(lpm_handle* h, const SellView& sv, const MixedGrids& mg) {
   cudaGraphNode_t wnode;
   LPM_CUDA(h, cudaGraphAddNode(&wnode, g, nullptr, nullptr, 0, &wp));
   cudaGraph_t body = wp.conditional.phGraph_out[0];
-  LPM_CUDA(h, cudaGraphConditionalHandleCreate(&ru_cond, body, 0u, cudaGraphCondAssignDefault));
-  cudaGraphNode_t n_spmv, n_upd, n_if, n_res, n_rep, n_pup;
-  cudaError_t e;
   const Spmv32Fn spmv = h->mf ? nullptr : spmv32_fn(h, sv);
-  if (h->mf) {
-    const int st = mf_graph_product(h, body, nullptr, true, d.p32, d.q32, d.q32lo, &n_spmv);
-    if (st) return st;
-  } else {
-    LPM_CUDA(h, add_kernel(&n_spmv, body, nullptr, spmv, mg.spmv, 256, sv, (const float*)d.A32, (const float*)d.p32,
-                           d.q32, d.cg, d.red.partials, d.red.ticket + 3, d.q32lo));
+  cudaGraphNode_t n_pup;
+  for (int k = 0; k < kGraphIterations; ++k) {
+    const cudaGraphNode_t before = n_pup, *after = k > 0 ? &before : nullptr;
+    const bool last = k + 1 == kGraphIterations;
+    cudaGraphConditionalHandle ru_cond;
+    LPM_CUDA(h, cudaGraphConditionalHandleCreate(&ru_cond, body, 0u, cudaGraphCondAssignDefault));
+    cudaGraphNode_t n_spmv, n_upd, n_if, n_res, n_rep;
+    cudaError_t e;
+    if (h->mf) {
+      const int st = mf_graph_product(h, body, after, true, d.p32, d.q32, d.q32lo, &n_spmv);
+      if (st) return st;
+    } else {
+      LPM_CUDA(h, add_kernel(&n_spmv, body, after, spmv, mg.spmv, 256, sv, (const float*)d.A32, (const float*)d.p32,
+                             d.q32, d.cg, d.red.partials, d.red.ticket + 3, d.q32lo));
+    }
+    LPM_CUDA(h, add_kernel(&n_upd, body, &n_spmv, k_mx_update, mg.update, 256, ndof, d.x32, d.x32lo, d.r32, d.r32lo,
+                           (const float*)d.p32, (const float*)d.q32, (const float*)d.q32lo, (const float*)d.invd32,
+                           d.cg, d.red.partials, d.red.ticket + 4, ru_cond));
+    cudaGraphNodeParams ip = {};
+    ip.type = cudaGraphNodeTypeConditional;
+    ip.conditional.handle = ru_cond;
+    ip.conditional.type = cudaGraphCondTypeIf;
+    ip.conditional.size = 1;
+    LPM_CUDA(h, cudaGraphAddNode(&n_if, body, &n_upd, nullptr, 1, &ip));
+    cudaGraph_t ifb = ip.conditional.phGraph_out[0];
+    if (h->mf) {
+      const int st = mf_graph_residual(h, ifb, nullptr, &n_res);
+      if (st) return st;
+      e = cudaSuccess;
+    } else if (dim == 3)
+      e = add_kernel(&n_res, ifb, nullptr, k_mx_residual<3>, mg.residual, 256, sv, (const double*)d.A64, (const double*)d.x64,
+                     (const float*)d.x32, (const float*)d.x32lo, (const double*)d.rhs, d.r64, d.cg, d.red.partials,
+                     d.red.ticket + 6);
+    else
+      e = add_kernel(&n_res, ifb, nullptr, k_mx_residual<2>, mg.residual, 256, sv, (const double*)d.A64, (const double*)d.x64,
+                     (const float*)d.x32, (const float*)d.x32lo, (const double*)d.rhs, d.r64, d.cg, d.red.partials,
+                     d.red.ticket + 6);
+    LPM_CUDA(h, e);
+    LPM_CUDA(h, add_kernel(&n_rep, ifb, &n_res, k_mx_replace, mg.replace, 256, ndof, (const double*)d.r64, d.r32, d.r32lo,
+                           d.x32, d.x32lo, d.x64, (const float*)d.p32, (const float*)d.invd32, d.cg, d.red.partials,
+                           d.red.ticket + 7));
+    LPM_CUDA(h, add_kernel(&n_pup, body, &n_if, k_mx_pupdate, mg.pupdate, 256, ndof, (const float*)d.r32,
+                           (const float*)d.invd32, d.p32, d.cg, last ? loop_cond : 0));
   }
-  LPM_CUDA(h, add_kernel(&n_upd, body, &n_spmv, k_mx_update, mg.update, 256, ndof, d.x32, d.x32lo, d.r32, d.r32lo,
-                         (const float*)d.p32, (const float*)d.q32, (const float*)d.q32lo, (const float*)d.invd32,
-                         d.cg, d.red.partials, d.red.ticket + 4, ru_cond));
-  cudaGraphNodeParams ip = {};
-  ip.type = cudaGraphNodeTypeConditional;
-  ip.conditional.handle = ru_cond;
-  ip.conditional.type = cudaGraphCondTypeIf;
-  ip.conditional.size = 1;
-  LPM_CUDA(h, cudaGraphAddNode(&n_if, body, &n_upd, nullptr, 1, &ip));
-  cudaGraph_t ifb = ip.conditional.phGraph_out[0];
-  if (h->mf) {
-    const int st = mf_graph_residual(h, ifb, nullptr, &n_res);
-    if (st) return st;
-    e = cudaSuccess;
-  } else if (dim == 3)
-    e = add_kernel(&n_res, ifb, nullptr, k_mx_residual<3>, mg.residual, 256, sv, (const double*)d.A64, (const double*)d.x64,
-                   (const float*)d.x32, (const float*)d.x32lo, (const double*)d.rhs, d.r64, d.cg, d.red.partials,
-                   d.red.ticket + 6);
-  else
-    e = add_kernel(&n_res, ifb, nullptr, k_mx_residual<2>, mg.residual, 256, sv, (const double*)d.A64, (const double*)d.x64,
-                   (const float*)d.x32, (const float*)d.x32lo, (const double*)d.rhs, d.r64, d.cg, d.red.partials,
-                   d.red.ticket + 6);
-  LPM_CUDA(h, e);
-  LPM_CUDA(h, add_kernel(&n_rep, ifb, &n_res, k_mx_replace, mg.replace, 256, ndof, (const double*)d.r64, d.r32, d.r32lo,
-                         d.x32, d.x32lo, d.x64, (const float*)d.p32, (const float*)d.invd32, d.cg, d.red.partials,
-                         d.red.ticket + 7));
-  LPM_CUDA(h, add_kernel(&n_pup, body, &n_if, k_mx_pupdate, mg.pupdate, 256, ndof, (const float*)d.r32,
-                         (const float*)d.invd32, d.p32, d.cg, loop_cond));
   LPM_CUDA(h, cudaGraphInstantiate(&h->mx_exec, g, 0));
   h->mx_graph_spmv = (const void*)spmv;
   h->mx_graph_mf = h->mf;
@@ -1534,7 +1554,7 @@ int build_mixed_graph(lpm_handle* h, const SellView& sv, const MixedGrids& mg) {
 }
 
 // The FP64 solve's iteration loop as one graph:
-//   while (loop_cond) { spmv; update; pupdate }
+//   while (loop_cond) { kGraphIterations times: spmv; update; pupdate }
 // with pupdate setting loop_cond once update has decided (converged,
 // iteration cap or non-finite).
 int build_fp64_graph(lpm_handle* h, const double* A, const double* b, double* x, double* r, double* p, double* q,
@@ -1559,20 +1579,24 @@ int build_fp64_graph(lpm_handle* h, const double* A, const double* b, double* x,
   cudaGraphNode_t wnode, n_spmv, n_upd, n_pup;
   LPM_CUDA(h, cudaGraphAddNode(&wnode, g, nullptr, nullptr, 0, &wp));
   cudaGraph_t body = wp.conditional.phGraph_out[0];
-  if (h->mf) {
-    const int st = mf_graph_product(h, body, nullptr, false, p, q, nullptr, &n_spmv);
-    if (st) return st;
-  } else if (h->dim == 3) {
-    LPM_CUDA(h, add_kernel(&n_spmv, body, nullptr, k_cg_spmv<double, 3>, GR, 256, sv, A, (const double*)p, q, d.cg,
-                           d.red.partials, d.red.ticket + 3, (float*)nullptr));
-  } else {
-    LPM_CUDA(h, add_kernel(&n_spmv, body, nullptr, k_cg_spmv<double, 2>, GR, 256, sv, A, (const double*)p, q, d.cg,
-                           d.red.partials, d.red.ticket + 3, (float*)nullptr));
+  for (int k = 0; k < kGraphIterations; ++k) {
+    const cudaGraphNode_t before = n_pup, *after = k > 0 ? &before : nullptr;
+    const bool last = k + 1 == kGraphIterations;
+    if (h->mf) {
+      const int st = mf_graph_product(h, body, after, false, p, q, nullptr, &n_spmv);
+      if (st) return st;
+    } else if (h->dim == 3) {
+      LPM_CUDA(h, add_kernel(&n_spmv, body, after, k_cg_spmv<double, 3>, GR, 256, sv, A, (const double*)p, q, d.cg,
+                             d.red.partials, d.red.ticket + 3, (float*)nullptr));
+    } else {
+      LPM_CUDA(h, add_kernel(&n_spmv, body, after, k_cg_spmv<double, 2>, GR, 256, sv, A, (const double*)p, q, d.cg,
+                             d.red.partials, d.red.ticket + 3, (float*)nullptr));
+    }
+    LPM_CUDA(h, add_kernel(&n_upd, body, &n_spmv, k_cg_update<double>, GV, 256, ndof, x, r, (const double*)p,
+                           (const double*)q, invd, d.cg, d.red.partials, d.red.ticket + 4));
+    LPM_CUDA(h, add_kernel(&n_pup, body, &n_upd, k_cg_pupdate<double>, GV, 256, ndof, (const double*)r, invd, p, d.cg,
+                           last ? loop_cond : 0));
   }
-  LPM_CUDA(h, add_kernel(&n_upd, body, &n_spmv, k_cg_update<double>, GV, 256, ndof, x, r, (const double*)p,
-                         (const double*)q, invd, d.cg, d.red.partials, d.red.ticket + 4));
-  LPM_CUDA(h, add_kernel(&n_pup, body, &n_upd, k_cg_pupdate<double>, GV, 256, ndof, (const double*)r, invd, p, d.cg,
-                         loop_cond));
   LPM_CUDA(h, cudaGraphInstantiate(&h->fp_exec, g, 0));
   h->fp_graph_x = x;
   h->fp_graph_mf = h->mf;
@@ -1791,7 +1815,7 @@ int solve_mixed(lpm_handle* h, double tol, long long maxit, long long* iters, do
       return LPM_ERR_STATE;
     }
   } else if (!timing) {
-    h->stats.kernel_launches += 3 * c.graph_passes + 2 * c.ru_count;
+    h->stats.kernel_launches += 3 * kGraphIterations * c.graph_passes + 2 * c.ru_count;
   }
   if (timing) {
     double ms_sum = 0.0;

@@ -53,7 +53,7 @@ struct CgScalars {
   int pfault;         // persistent solve: a grid-barrier wait gave up
   double rmax;        // mixed solve: largest |r| since the last reliable update
   long long ru_count; // mixed solve: reliable updates taken
-  long long graph_passes;  // mixed solve: loop passes run by the solve graph
+  long long graph_passes;  // loop passes run by a solve graph (kGraphIterations each), or a persistent solve's iterations
   double zcoef;       // mixed solve: p = zcoef z + beta p (1 except right after an update)
   unsigned long long bmax_bits;  // mixed solve: bits of max |b| (non-negative doubles order as integers)
   double bscale;      // mixed solve: power of two that brings max |b| to [1, 2)
