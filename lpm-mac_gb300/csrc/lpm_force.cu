@@ -5,8 +5,6 @@
 // take its bonds in stored order in turn (Particle::bond_layers,
 // particle.h:163-181, 197-240); a bond's own values are the same with any
 // number of lanes, a particle's sums are the lanes' added in a fixed order.
-#include <climits>
-
 #include "lpm_device.cuh"
 
 namespace lpm {
@@ -353,7 +351,7 @@ int launch_geometry_force(lpm_handle* h) {
   // 5,210, 7,379.  So four up to 200 threads on each of the 152 SMs, two up to
   // all they hold.
   const int L = h->n <= 7600 ? 4 : h->n <= 155000 ? 2 : 1;
-  const int T = 128, G = grid_for((long long)h->n * L, T, INT_MAX);
+  const int T = 128, G = grid_for((long long)h->n * L, T);
   const auto geometry = L == 4 ? k_geometry_force<4> : L == 2 ? k_geometry_force<2> : k_geometry_force<1>;
   const auto particle = L == 4 ? k_particle_force<4> : L == 2 ? k_particle_force<2> : k_particle_force<1>;
   geometry<<<G, T, 0, h->stream>>>(h->n, d.x, d.bptr, d.bp2, d.blayer, d.dis0, d.dLp, d.bdamage, d.Kn, d.Tv, d.dis,

@@ -26,6 +26,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include <string>
@@ -374,7 +375,9 @@ int cuda_fail(lpm_handle* h, cudaError_t e, const char* what);
 void set_global_error(const std::string& msg);  // text of lpm_last_error(NULL)
 void* dev_alloc(lpm_handle* h, size_t bytes);
 void* zeros_dev(lpm_handle* h, size_t bytes);  // dev_alloc + zero fill
-inline int grid_for(long long work, int threads, int cap = 1 << 20) {
+// Blocks for `work` threads.  No cap unless the kernel loops with a grid stride:
+// one that does not would leave out what lies past it.
+inline int grid_for(long long work, int threads, int cap = INT_MAX) {
   long long g = (work + threads - 1) / threads;
   if (g < 1) g = 1;
   if (g > cap) g = cap;

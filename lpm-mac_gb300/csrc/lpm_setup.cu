@@ -11,7 +11,6 @@
 // lattice) put in input order by one thread; 0.2 ms together.  Bound by the
 // copy of the list to the device.
 #include <algorithm>
-#include <climits>
 
 #include "lpm_device.cuh"
 
@@ -207,7 +206,7 @@ int build_bonds(lpm_handle* h, const int* p1, const int* p2, const int* layer, c
       LPM_CUDA(h, cudaMemcpyAsync(kn, Kn, sizeof(double) * nb, cudaMemcpyHostToDevice, h->stream));
       LPM_CUDA(h, cudaMemcpyAsync(tv, Tv, sizeof(double) * nb, cudaMemcpyHostToDevice, h->stream));
     }
-    const int GB = grid_for(nb, T, INT_MAX), GM = grid_for(m, T, INT_MAX);
+    const int GB = grid_for(nb, T), GM = grid_for(m, T);
     k_bond_count<<<GB, T, 0, h->stream>>>(nb, q1, ql, cnt);
     LPM_LAUNCHED(h, "k_bond_count");
     k_scan_blocks<<<blocks, kScan, 0, h->stream>>>(m, cnt, at, sums);
@@ -227,7 +226,7 @@ int build_bonds(lpm_handle* h, const int* p1, const int* p2, const int* layer, c
     LPM_LAUNCHED(h, "k_bond_opposite");
     k_bond_sorted<<<GM, T, 0, h->stream>>>(m, nb, at, d.bp2, d.sbond, d.sp2, d.nbonds);
     LPM_LAUNCHED(h, "k_bond_sorted");
-    k_ones<<<grid_for(n, T, INT_MAX), T, 0, h->stream>>>(n, d.crit, d.pp);
+    k_ones<<<grid_for(n, T), T, 0, h->stream>>>(n, d.crit, d.pp);
     LPM_LAUNCHED(h, "k_ones");
     int bad = 0;
     LPM_CUDA(h, cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
