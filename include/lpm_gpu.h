@@ -298,6 +298,8 @@ typedef struct {
 } lpm_stats;
 int lpm_get_stats(const lpm_handle* h, lpm_stats* st);
 int lpm_reset_stats(lpm_handle* h);
+/* Of persistent_solves, those that ran on chip (lpm_set_cg_loop). */
+int lpm_get_onchip_solves(const lpm_handle* h, int64_t* n);
 /* Records CUDA events around every CG sparse-product launch (on the
  * handle's stream) so that lpm_get_stats reports its device time.  While it
  * is on, the solves launch their iterations one by one from the host instead

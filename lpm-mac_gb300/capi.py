@@ -139,6 +139,7 @@ def load(build_if_needed=True):
         "lpm_reset_state": [H, ctypes.c_int],
         "lpm_get_stats": [H, ctypes.POINTER(Stats)],
         "lpm_reset_stats": [H],
+        "lpm_get_onchip_solves": [H, i64p],
         "lpm_set_kernel_timing": [H, ctypes.c_int],
         "lpm_set_cg_loop": [H, ctypes.c_int],
         "lpm_set_preconditioner": [H, ctypes.c_int, ctypes.c_double],
@@ -181,7 +182,7 @@ def exported_symbols():
             "lpm_update_geometry_force", "lpm_residual", "lpm_assemble", "lpm_get_K", "lpm_set_operator",
             "lpm_apply_operator", "lpm_solve",
             "lpm_move_by_disp", "lpm_newton", "lpm_load_step", "lpm_store_state", "lpm_reset_state",
-            "lpm_get_stats", "lpm_reset_stats", "lpm_set_kernel_timing", "lpm_set_cg_loop", "lpm_set_preconditioner", "lpm_coarse_boxes", "lpm_get_stream", "lpm_synchronize",
+            "lpm_get_stats", "lpm_reset_stats", "lpm_get_onchip_solves", "lpm_set_kernel_timing", "lpm_set_cg_loop", "lpm_set_preconditioner", "lpm_coarse_boxes", "lpm_get_stream", "lpm_synchronize",
             "lpm_find_bonds", "lpm_find_neighbors", "lpm_fatigue_cycle", "lpm_fatigue_run", "lpm_backward_step", "lpm_apply_jacobian", "lpm_checkpoint_save", "lpm_checkpoint_restore",
             "lpm_checkpoint_drop", "lpm_tangent_begin", "lpm_tangent_bond_constants", "lpm_tangent_bond_scrit",
             "lpm_tangent_get",
@@ -525,6 +526,12 @@ class Lattice:
 
     def reset_stats(self):
         self._check(self._L.lpm_reset_stats(self.h))
+
+    def onchip_solves(self):
+        """Of stats()["persistent_solves"], those that ran on chip."""
+        n = ctypes.c_int64()
+        self._check(self._L.lpm_get_onchip_solves(self.h, ctypes.byref(n)))
+        return n.value
 
     def set_cg_loop(self, mode):
         """CG_LOOP_AUTO (default), CG_LOOP_GRAPH or CG_LOOP_PERSISTENT: how the

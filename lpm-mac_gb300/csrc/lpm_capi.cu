@@ -745,9 +745,16 @@ int lpm_get_stats(const lpm_handle* h, lpm_stats* st) {
   return LPM_OK;
 }
 
+int lpm_get_onchip_solves(const lpm_handle* h, int64_t* n) {
+  if (!h || !n) return LPM_ERR_ARG;
+  *n = h->onchip_solves;
+  return LPM_OK;
+}
+
 int lpm_reset_stats(lpm_handle* h) {
   if (!h) return LPM_ERR_ARG;
   h->stats = lpm_stats{};
+  h->onchip_solves = 0;
   return LPM_OK;
 }
 

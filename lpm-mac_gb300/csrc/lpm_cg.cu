@@ -1230,7 +1230,10 @@ int run_persistent_fp64(lpm_handle* h, const SellView& sv, const double* A, doub
   if (!h->mf && h->cg_loop != LPM_CG_LOOP_GRAPH) {  // on chip where one wave of blocks holds the rows
     const int st = pcg_run_fp64(h, A, x, r, invd, (long long)h->nslots * h->dim * h->dim * 8 <= kKeepBytes);
     if (st < 0) return st;
-    if (st == 1) return persistent_done(h);
+    if (st == 1) {
+      h->onchip_solves += 1;
+      return persistent_done(h);
+    }
   }
   using Fn = void (*)(PcgFp64);
   const Fn fn = h->dim == 3 ? k_cg_persistent<3> : k_cg_persistent<2>;
@@ -1810,6 +1813,7 @@ int solve_mixed(lpm_handle* h, double tol, long long maxit, long long* iters, do
   const CgScalars& c = *h->h_cg;
   if (pgrid > 0) {
     h->stats.persistent_solves += 1;
+    h->onchip_solves += on_chip;
     if (c.pfault) {
       h->err = "persistent solve: a grid-barrier wait gave up";
       return LPM_ERR_STATE;

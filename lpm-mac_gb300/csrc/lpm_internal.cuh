@@ -266,6 +266,7 @@ struct lpm_handle {
   lpm::CgScalars* h_cg = nullptr;  // pinned
   double* h_norms = nullptr;       // pinned [8]
   lpm_stats stats{};
+  int64_t onchip_solves = 0;  // of stats.persistent_solves, those of lpm_pcg.cu and lpm_pcg64.cu
   bool timing = false;
   int cg_loop = LPM_CG_LOOP_AUTO;  // how the solves run their iteration loop (lpm_set_cg_loop)
   int precond = LPM_PRECOND_JACOBI;  // preconditioner of the mixed solve (lpm_set_preconditioner)
