@@ -1,6 +1,8 @@
 """Which kernel a solve runs in, and the solve in each: on chip (k_pcg_mixed,
 k_pcg_fp64) with every number of slices to a block that changes the split of
-its work.  A solve is held to its stopping rule on the operator in FP64, |b - A x| <= tol |b| plus the
+its work, at grid barriers (k_mx_persistent, k_cg_persistent) past the on-chip
+solves' limits, the graph loop's product on 32-bit columns.  A solve is held to
+its stopping rule on the operator in FP64, |b - A x| <= tol |b| plus the
 rounding of forming the residual, 1e-13 |A| |x|, and its iterations to the graph
 loop's (5 % and four: the sums are folded in another order)."""
 import numpy as np
@@ -101,5 +103,43 @@ def test_on_chip_with_several_slices_a_block(name, precision):
     it, persistent, on_chip = s.solve(precision)
     assert (persistent, on_chip) == (1, 1)
     graph, persistent, on_chip = s.solve(precision, capi.CG_LOOP_GRAPH)
+    assert (persistent, on_chip) == (0, 0) and _like(it, graph)
+    s.g.close()
+
+
+@pytest.mark.parametrize("dim,size,precision", [(2, (250, 245), FP64),    # 13 slices: k_cg_persistent
+                                                (3, (40, 40, 40), FP64),  # 14
+                                                (2, (345, 345), MIXED),   # 25: k_mx_persistent
+                                                (3, (43, 43, 43), MIXED)])  # 17
+def test_grid_barrier_solve_past_the_on_chip_limits(dim, size, precision):
+    s = System(_body(dim, size))
+    it, persistent, on_chip = s.solve(precision, capi.CG_LOOP_PERSISTENT)
+    assert (persistent, on_chip) == (1, 0)
+    graph, persistent, on_chip = s.solve(precision, capi.CG_LOOP_GRAPH)
+    assert (persistent, on_chip) == (0, 0) and _like(it, graph)
+    s.g.close()
+
+
+@pytest.mark.parametrize("dim,size", [(2, (345, 345)), (3, (43, 43, 43))])
+def test_grid_barrier_coarse_solve_past_the_on_chip_limits(dim, size):
+    """k_mx_persistent with the coarse correction: its residual, and fewer
+    iterations than without."""
+    s = System(_body(dim, size), capi.PRECOND_COARSE)
+    it, persistent, on_chip = s.solve(MIXED)
+    assert (persistent, on_chip) == (1, 0)
+    s.g.set_preconditioner(capi.PRECOND_JACOBI)
+    assert it < 0.7 * s.solve(MIXED, capi.CG_LOOP_GRAPH)[0]
+    s.g.close()
+
+
+@pytest.mark.parametrize("dim,size", [(2, (190, 190)), (3, (33, 33, 33))])
+def test_graph_loop_on_32_bit_columns(dim, size):
+    """Columns further than 16 bits from their rows: the graph loop's FP32
+    product on 32-bit columns, against the same solve on chip."""
+    s = System(_body(dim, size, 10**9))
+    assert s.reach > 32767
+    it, persistent, on_chip = s.solve(MIXED)
+    assert (persistent, on_chip) == (1, 1)
+    graph, persistent, on_chip = s.solve(MIXED, capi.CG_LOOP_GRAPH)
     assert (persistent, on_chip) == (0, 0) and _like(it, graph)
     s.g.close()
