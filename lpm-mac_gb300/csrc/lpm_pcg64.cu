@@ -556,12 +556,25 @@ __global__ void __launch_bounds__(kPcg64Threads, 1) k_pcg_fp64(const __grid_cons
     for (int k = 0; k < DIM; ++k) a.r[i0 + k] = r[k];
 }
 
+// Most columns a row (of the largest block) in 2-D with more than nine slices:
+// where the numbering scatters a row's neighbours every block forms p at nearly
+// all the columns its rows name, and k_cg_persistent, which forms p once, is
+// ahead.  us per iteration of plates numbered at random (28 columns a row),
+// here against there: 44k rows, ten slices, 34.1 (31.7), 45.9k 34.4 (31.6), 50.3k,
+// eleven, 37.8 (32.8), 52k 38.0 (32.3); within windows of 16,384 particles (24 to 27
+// columns) the two are even, 45.9k 31.7 (31.6), or this is ahead, 57.8k 31.9
+// (34.8).  Up to nine slices it depends on the box: 23.7k rows 23.0 (24.5), 33.9k
+// 28.8 (29.1 to 29.7), 39.8k 29.3 or 32.1 (30.7).  In 3-D, nine elements to a block,
+// what fits is ahead: 26^3 at random, 47 columns a row, 37.4 (69.4).
+constexpr int kColumnsPerRow = 26, kColumnsSlices = 9;
+
 // Launch shape, once per handle: the staged vector, its columns, the partial
 // sums, the diagonal, the slices' tail blocks and as many groups of each
 // warp as fit.
 template <int DIM>
 bool shape64(const lpm_handle* h, const void* fn, PcgShape* sh) {
   const PcgPlan& pl = h->pcg;
+  if (DIM == 2 && pl.S > kColumnsSlices && pl.umax > kColumnsPerRow * kSlice * pl.S) return false;
   auto align = [](size_t b) { return (int)((b + 15) / 16 * 16); };
   const int W = fp64_warps(DIM, pl.S);
   int tails = 0, most = 0;  // most tail blocks of a slice, most groups of a block

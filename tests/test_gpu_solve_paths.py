@@ -107,6 +107,20 @@ def test_on_chip_with_several_slices_a_block(name, precision):
     s.g.close()
 
 
+@pytest.mark.parametrize("size,window,on_chip", [((190, 210), 10**9, 1),  # 9 slices, 28.0 columns a row
+                                                 ((200, 230), 10**9, 0),  # 10, 28.1
+                                                 ((200, 230), 4096, 1)])  # 10, 18.6
+def test_fp64_solve_of_scattered_numberings(size, window, on_chip):
+    """On chip in 2-D up to 26 columns a row where a block has more than nine
+    slices (past that k_cg_persistent is the faster); the mixed solve always."""
+    s = System(_body(2, size, window))
+    it, persistent, here = s.solve(FP64)
+    assert (persistent, here) == (1, on_chip)
+    assert _like(it, s.solve(FP64, capi.CG_LOOP_GRAPH)[0])
+    assert s.solve(MIXED)[1:] == (1, 1)
+    s.g.close()
+
+
 @pytest.mark.parametrize("dim,size,precision", [(2, (250, 245), FP64),    # 13 slices: k_cg_persistent
                                                 (3, (40, 40, 40), FP64),  # 14
                                                 (2, (345, 345), MIXED),   # 25: k_mx_persistent
