@@ -292,7 +292,9 @@ typedef struct {
   double spmv32_ms;
   int64_t kernel_launches;
   int64_t mixed_fallbacks; /* mixed solves that broke down (non-finite FP32 recurrence,
-                              e.g. an indefinite softened tangent) and were re-solved in FP64 */
+                              e.g. an indefinite softened tangent, or r.z outside FP32's range:
+                              bond constants past 1e15 at a tolerance of 1e-13, 1e21 at 1e-10)
+                              and were re-solved in FP64 */
   int64_t tangent_cg_iters; /* CG iterations of the tangent solves (lpm_tangent_begin) */
   int64_t persistent_solves; /* solves whose loop ran as one persistent kernel (lpm_set_cg_loop) */
 } lpm_stats;

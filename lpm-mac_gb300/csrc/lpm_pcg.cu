@@ -251,7 +251,12 @@ __device__ __forceinline__ PcgShared& block_state() { return *reinterpret_cast<P
 __device__ __forceinline__ float* staged_p(const PcgMixedArgs& a) { return reinterpret_cast<float*>(dyn + a.off_p); }
 
 // (qh, ql) = (ah, al) / (bh, bl): quotient digits of FP32 from the reciprocal,
-// each with its remainder by FMA (long division); about 2^-46.
+// each with its remainder by FMA (long division); about 2^-46.  A divisor below
+// 2.9e-39 has no FP32 reciprocal: the quotient is not finite, the solve ends as
+// broken down (done = 3) and runs again in FP64.  r.z and p.q go with the inverse of
+// the stiffness, so that is where a solve of constants past 1e15 at a tolerance
+// of 1e-13, or 1e21 at 1e-10, ends.  Scaled into range here such solves went on
+// with rows' products of few or no digits, and some never converged.
 __device__ __forceinline__ void df_div(float ah, float al, float bh, float bl, float& qh, float& ql) {
   const float rc = __frcp_rn(bh);
   const float q1 = __fmul_rn(ah, rc);
