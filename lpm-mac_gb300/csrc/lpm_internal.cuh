@@ -223,7 +223,8 @@ struct PcgPlan {
   int state = 0;  // 0 not made, 1 usable, -1 not
   PcgShape mixed, mixed_coarse, fp64;
   int cmaxagg = 0, centries = 0;  // coarse correction: most aggregates a block's rows touch, (block, aggregate) pairs
-  int G = 0, S = 0, umax = 0, smem = 0;  // blocks, slices of the largest, most columns of one, shared memory of an SM
+  int G = 0, S = 0, umax = 0, smem = 0;  // blocks, slices of the largest, most columns of one, most shared memory of a block
+  int half = 0;                          // most of a block where an SM is to hold two
 };
 
 // One device-resident copy of a step's state (lpm_checkpoint_save).

@@ -1244,10 +1244,13 @@ int pcg_plan(lpm_handle* h) {
   if (pl.state) return pl.state > 0;
   pl.state = -1;
   Dev& d = h->d;
-  int coop = 0, smem = 0;
+  int coop = 0, smem = 0, sm_smem = 0, reserved = 0;
   if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device) != cudaSuccess || !coop) return 0;
   if (!h->sms && cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) return 0;
-  if (cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device) != cudaSuccess) return 0;
+  if (cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, h->device) != cudaSuccess)
+    return 0;
   const int G = std::min(std::min(h->sms, kPcgMaxBlocks), h->nslice);
   const int S = (h->nslice + G - 1) / G;
   if (S > kPcgMaxSlices) return 0;
@@ -1280,6 +1283,7 @@ int pcg_plan(lpm_handle* h) {
   pl.S = S;
   pl.umax = umax;
   pl.smem = smem;
+  pl.half = sm_smem / 2 - reserved;
   pl.state = 1;
   return 1;
 }
@@ -1294,10 +1298,11 @@ size_t align16(size_t b) { return (b + 15) / 16 * 16; }
 // `unit` is a group's bytes, `threads` the most per block, `vec` the bytes of
 // a staged entry, `part` of a row's partial sums of one share, `rowc` of a
 // row's constants, `coarse` of the coarse correction.
-bool shape_on_plan(const lpm_handle* h, const void* fn, int threads, size_t unit, size_t vec, size_t part,
-                   size_t rowc, size_t coarse, PcgShape* sh) {
+// maxw compute warps and smem bytes at most; `share`: only if all groups fit, in
+// blocks of which an SM holds two.
+bool shape_with(const lpm_handle* h, const void* fn, int maxw, int smem, bool share, size_t unit, size_t vec,
+                size_t part, size_t rowc, size_t coarse, PcgShape* sh) {
   const PcgPlan& pl = h->pcg;
-  const int maxw = threads / 32 - 1;  // compute warps
   if (pl.S > maxw) return false;
   auto groups = [&](int s) {
     const int w = (int)((h->sell_host[(size_t)s + 1] - h->sell_host[(size_t)s]) / kSlice);
@@ -1312,7 +1317,7 @@ bool shape_on_plan(const lpm_handle* h, const void* fn, int threads, size_t unit
   sh->off_row = sh->off_part + (int)align16(part * (size_t)(sh->T - 1) * pl.S * 32);
   sh->off_coarse = sh->off_row + (int)align16(rowc * (size_t)pl.S * 32);
   sh->off_op = sh->off_coarse + (int)align16(coarse);
-  const long long room = (long long)pl.smem - sh->off_op;
+  const long long room = (long long)smem - sh->off_op;
   if (room < 0) return false;
   size_t units = 0;
   sh->gs = sh->gx = 0;
@@ -1333,17 +1338,36 @@ bool shape_on_plan(const lpm_handle* h, const void* fn, int threads, size_t unit
       sh->gx = x;
       units = most;
     }
+  if (share && sh->gs + (sh->gx == pl.S ? 1 : 0) < gmax) return false;
   sh->bytes = (size_t)sh->off_op + units * unit;
-  sh->threads = (pl.S * sh->T + 1) * 32;
+  // (warps without a share still take their part in the coarse correction)
+  sh->threads = (share && coarse ? maxw + 1 : pl.S * sh->T + 1) * 32;
   int per_sm = 0;
   // (the attribute belongs to the kernel, not to the handle: always the most)
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, sh->threads, sh->bytes) != cudaSuccess ||
-      per_sm < 1) {
+      per_sm < (share ? 2 : 1)) {
     cudaGetLastError();
     return false;
   }
   return true;
+}
+
+// Once per handle.  Blocks of up to two slices take seven compute warps at most
+// and half an SM, where their groups fit it, so that the solves of several small
+// systems, from several threads, run beside each other; with fifteen warps they
+// took turns.  us per iteration alone, with fifteen warps and with seven: a 41x41
+// plate 7.1 and 7.2, 61x121 7.1 and 6.9, a 12^3 cube 9.7 and 9.6; of four handles
+// solved at once (over all their iterations) 3.5 and 1.9, 7.0 and 3.7, 4.7 and 2.8.
+// (With k_mx_persistent, whose blocks are smaller still, 4.2, 4.3 and 7.6.)
+constexpr int kSharingWarps = 7;
+
+bool shape_on_plan(const lpm_handle* h, const void* fn, int threads, size_t unit, size_t vec, size_t part,
+                   size_t rowc, size_t coarse, PcgShape* sh) {
+  const PcgPlan& pl = h->pcg;
+  return (pl.S <= kSharingSlices &&
+          shape_with(h, fn, kSharingWarps, pl.half, true, unit, vec, part, rowc, coarse, sh)) ||
+         shape_with(h, fn, threads / 32 - 1, pl.smem, false, unit, vec, part, rowc, coarse, sh);
 }
 
 template <int DIM, bool COARSE>

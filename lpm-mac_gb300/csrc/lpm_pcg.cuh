@@ -71,6 +71,9 @@ constexpr int kPcg64Slices = 12;
 __host__ __device__ __forceinline__ int fp64_warps(int dim, int S) {
   return dim == 3 ? kPcg64Slices : S <= 8 ? 8 : kPcg64Slices;
 }
+// Most slices of a block whose launch leaves room for a second block on its SM
+// (shape_on_plan, shape64).
+constexpr int kSharingSlices = 2;
 // Threads per block of the FP64 solve, at most, the message warp included
 // (128 registers).
 constexpr int kPcg64Threads = 512;

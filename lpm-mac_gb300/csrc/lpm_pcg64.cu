@@ -568,15 +568,14 @@ __global__ void __launch_bounds__(kPcg64Threads, 1) k_pcg_fp64(const __grid_cons
 // what fits is ahead: 26^3 at random, 47 columns a row, 37.4 (69.4).
 constexpr int kColumnsPerRow = 26, kColumnsSlices = 9;
 
-// Launch shape, once per handle: the staged vector, its columns, the partial
-// sums, the diagonal, the slices' tail blocks and as many groups of each
-// warp as fit.
+// Launch shape with W compute warps in smem bytes: the staged vector, its
+// columns, the partial sums, the diagonal, the slices' tail blocks and as many
+// groups of each warp as fit.  `share`: only if all of them do, in blocks of which
+// an SM holds two.
 template <int DIM>
-bool shape64(const lpm_handle* h, const void* fn, PcgShape* sh) {
+bool shape64_with(const lpm_handle* h, const void* fn, int W, int smem, bool share, PcgShape* sh) {
   const PcgPlan& pl = h->pcg;
-  if (DIM == 2 && pl.S > kColumnsSlices && pl.umax > kColumnsPerRow * kSlice * pl.S) return false;
   auto align = [](size_t b) { return (int)((b + 15) / 16 * 16); };
-  const int W = fp64_warps(DIM, pl.S);
   int tails = 0, most = 0;  // most tail blocks of a slice, most groups of a block
   for (int b = 0; b < pl.G; ++b) {
     int g = 0;
@@ -594,23 +593,39 @@ bool shape64(const lpm_handle* h, const void* fn, PcgShape* sh) {
   sh->off_row = sh->off_part + align(sizeof(double) * DIM * 32 * (size_t)(W + pl.S));
   sh->off_coarse = sh->off_row + align(sizeof(double) * DIM * 32 * (size_t)pl.S);  // the tail blocks
   const int tbytes = align((size_t)kPcgUnit64<DIM> / kVec * tails * (size_t)pl.S);
-  if (sh->off_coarse > pl.smem) return false;
-  sh->tails = sh->off_coarse + tbytes <= pl.smem ? tails : 0;
+  if (sh->off_coarse > smem) return false;
+  sh->tails = sh->off_coarse + tbytes <= smem ? tails : 0;
   sh->off_op = sh->off_coarse + (sh->tails ? tbytes : 0);
-  const int units = (pl.smem - sh->off_op) / kPcgUnit64<DIM>, need = (most + W - 1) / W;
+  const int units = (smem - sh->off_op) / kPcgUnit64<DIM>, need = (most + W - 1) / W;
   sh->gs = std::min(units / W, need);
   sh->gx = sh->gs < need ? units - sh->gs * W : 0;
+  if (share && (sh->gs < need || sh->tails < tails)) return false;
   sh->bytes = (size_t)sh->off_op + (size_t)(sh->gs * W + sh->gx) * kPcgUnit64<DIM>;
   sh->threads = (W + 1) * 32;
   int per_sm = 0;
   // (the attribute belongs to the kernel, not to the handle: always the most)
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, sh->threads, sh->bytes) != cudaSuccess ||
-      per_sm < 1) {
+      per_sm < (share ? 2 : 1)) {
     cudaGetLastError();
     return false;
   }
   return true;
+}
+
+// Once per handle.  Blocks of one slice take four warps and those of two seven,
+// and half an SM, where their groups fit it, so that the solves of several small
+// systems, from several threads, run beside each other.  us per iteration alone,
+// with eight warps and so: a 41x41 plate 11.1 and 11.3, 61x80 11.0 and 11.0, 61x121
+// 12.7 and 12.5, 75x110 11.7 and 12.3; of four handles solved at once (over all
+// their iterations) a 41x41 plate 5.2 and 3.0, 61x121 12.4 and 6.0.  (With
+// k_cg_persistent 5.4 and 7.1.)
+template <int DIM>
+bool shape64(const lpm_handle* h, const void* fn, PcgShape* sh) {
+  const PcgPlan& pl = h->pcg;
+  if (DIM == 2 && pl.S > kColumnsSlices && pl.umax > kColumnsPerRow * kSlice * pl.S) return false;
+  return (pl.S <= kSharingSlices && shape64_with<DIM>(h, fn, pl.S == 1 ? 4 : 7, pl.half, true, sh)) ||
+         shape64_with<DIM>(h, fn, fp64_warps(DIM, pl.S), pl.smem, false, sh);
 }
 
 template <int DIM>
