@@ -722,7 +722,7 @@ static int jacobian_cg(lpm_handle* h, const double* g, double* x, double tol, lo
   if (maxit < 0) maxit = 2LL * m;
   // two blocks per SM: the fold over the blocks of all of a 41^3 cube's DOFs
   // took 4 us of an iteration more
-  const int GV = grid_for(m, 256, h->sms > 0 ? std::min(2 * h->sms, kMaxRedBlocks) : kMaxRedBlocks);
+  const int GV = grid_for(m, 256, sm_count(h) > 0 ? std::min(2 * h->sms, kMaxRedBlocks) : kMaxRedBlocks);
   k_cg_init<double><<<GV, 256, 0, h->stream>>>(m, g, x, d.adj_r, d.adj_p, d.adj_invd, d.cg, tol, maxit,
                                                d.red.partials, d.red.ticket + 2);
   LPM_LAUNCHED(h, "k_cg_init");

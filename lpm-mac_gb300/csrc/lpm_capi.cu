@@ -22,6 +22,11 @@ int cuda_fail(lpm_handle* h, cudaError_t e, const char* what) {
   return e == cudaErrorMemoryAllocation ? LPM_ERR_NOMEM : LPM_ERR_CUDA;
 }
 
+int sm_count(lpm_handle* h) {
+  if (!h->sms && cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) h->sms = 0;
+  return h->sms;
+}
+
 void* dev_alloc(lpm_handle* h, size_t bytes) {
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 16));

@@ -1171,11 +1171,9 @@ int vec_grid(long long m) { return grid_for(m, 256, kMaxRedBlocks); }
 // cover any size.
 template <typename K>
 int resident_grid(lpm_handle* h, K kernel, long long work) {
-  if (!h->sms && cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess)
-    h->sms = 0;
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
-  const long long resident = h->sms > 0 ? (long long)h->sms * per_sm : kMaxRedBlocks;
+  const long long resident = sm_count(h) > 0 ? (long long)h->sms * per_sm : kMaxRedBlocks;
   const long long g = std::min<long long>(resident, (work + 255) / 256);
   return (int)std::max<long long>(1, std::min<long long>(g, kMaxRedBlocks));
 }
@@ -1192,7 +1190,7 @@ int persistent_shape(lpm_handle* h, K kernel, int cap, bool auto_ok, int slots, 
   if (h->mf || h->cg_loop == LPM_CG_LOOP_GRAPH) return 0;
   int coop = 0;
   if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device) != cudaSuccess || !coop) return 0;
-  if (!h->sms && cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) return 0;
+  if (!sm_count(h)) return 0;
   const long long per_sm_rows = ((long long)h->n + h->sms - 1) / h->sms;
   const int threads = (int)std::min<long long>(cap, std::max<long long>(128, (per_sm_rows + 31) / 32 * 32));
   *threads_out = threads;
@@ -1415,7 +1413,7 @@ Spmv32Fn spmv32_fn(const lpm_handle* h, const SellView& sv) {
 template <typename K>
 int vector_grid(lpm_handle* h, K kernel, long long ndof) {
   const int g = resident_grid(h, kernel, ndof);
-  const long long small = std::max<long long>(2LL * h->sms, (ndof + 1023) / 1024);
+  const long long small = std::max<long long>(2LL * sm_count(h), (ndof + 1023) / 1024);
   return (int)std::max<long long>(1, std::min<long long>(g, small));
 }
 

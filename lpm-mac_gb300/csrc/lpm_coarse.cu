@@ -514,10 +514,8 @@ int coarse_assemble(lpm_handle* h) {
                                                                   d.cA);
     LPM_LAUNCHED(h, "k_coarse_pairs");
   }
-  if (!h->sms && cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess)
-    h->sms = 1;
   // a block per SM: the barriers cost more with more
-  const int grid = std::max(1, h->sms);
+  const int grid = std::max(1, sm_count(h));
   LPM_CUDA(h, cudaMemsetAsync(d.gbar, 0, sizeof(unsigned long long), h->stream));
   LPM_CUDA(h, cudaMemsetAsync(d.cfault, 0, sizeof(int), h->stream));
   long long spin = kPcgSpinLimit;

@@ -257,7 +257,7 @@ struct lpm_handle {
   bool have_K = false;
   bool a32_valid = false;  // FP32 copy of the operator matches A64
   bool soff16_ok = false;  // every column offset of the pattern fits 16 bits
-  int sms = 0;             // multiprocessors of the device (looked up on the first mixed solve)
+  int sms = 0;             // multiprocessors of the device (sm_count)
   int tangent = LPM_TANGENT_AS_WRITTEN;
   bool mf = false;        // the CG applies the tangent matrix-free (lpm_set_operator)
   int64_t mslots = 0;     // slots of the matrix-free bond layout
@@ -375,6 +375,7 @@ int checkpoint_drop(lpm_handle* h, int id);
 // helpers (lpm_capi.cu)
 int cuda_fail(lpm_handle* h, cudaError_t e, const char* what);
 void set_global_error(const std::string& msg);  // text of lpm_last_error(NULL)
+int sm_count(lpm_handle* h);  // multiprocessors of the handle's device, looked up once; 0 if that fails
 void* dev_alloc(lpm_handle* h, size_t bytes);
 void* zeros_dev(lpm_handle* h, size_t bytes);  // dev_alloc + zero fill
 // Blocks for `work` threads.  No cap unless the kernel loops with a grid stride:
