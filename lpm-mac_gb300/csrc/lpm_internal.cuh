@@ -352,7 +352,7 @@ int prepare_invd(lpm_handle* h, bool want32);
 int apply_operator(lpm_handle* h, int precision, const double* v_host, double* y_host);
 // the solve's loop on chip (lpm_pcg.cu), its vectors initialised and its
 // scalars in d.cg: 1 launched, 0 not possible for this system, or an error
-int pcg_plan(lpm_handle* h);
+int pcg_plan(lpm_handle* h, int slices);
 int pcg_run_mixed(lpm_handle* h, bool keep, bool coarse);
 int pcg_run_fp64(lpm_handle* h, const double* A, double* x, double* r, const double* invd, bool keep);
 int pcg_coarse_plan(lpm_handle* h, const std::vector<int>& agg, int nagg);

@@ -53,7 +53,8 @@ namespace {
 constexpr int kPlanThreads = 256;
 // ------------------------------------------------------------------ plan
 // Columns of the block's slices as a bitmap over all particles, in shared
-// memory (n <= 2^17: 16 KB), and for each word the number of columns below it.
+// memory (at most 24 slices of 160 blocks, 122,880 particles: 15 KB), and for each
+// word the number of columns below it.
 __device__ void plan_bitmap(int n, int s0, int s1, const int64_t* __restrict__ sell_ptr,
                             const int* __restrict__ scol, const int* __restrict__ rowlen, unsigned* bits) {
   const int words = (n + 31) / 32;
@@ -1236,26 +1237,26 @@ static int pcg_no_memory(lpm_handle* h) {
   return 0;
 }
 
-// The column plan of the handle's pattern, once: 1 if the solves of this
-// file can run on it, 0 if not (more rows than one wave of blocks holds, or
-// no cooperative launch), or an error.
-int pcg_plan(lpm_handle* h) {
+// The column plan of the handle's pattern, once, for a solve of at most `slices`
+// to a block: 1 if it can run on the plan, 0 if not (more slices, or no
+// cooperative launch), or an error.
+int pcg_plan(lpm_handle* h, int slices) {
   PcgPlan& pl = h->pcg;
-  if (pl.state) return pl.state > 0;
+  if (pl.state) return pl.state > 0 && pl.S <= slices;
+  if (!sm_count(h)) return 0;
+  const int G = std::min(std::min(h->sms, kPcgMaxBlocks), h->nslice);
+  const int S = (h->nslice + G - 1) / G;
+  if (S > slices) return 0;
   pl.state = -1;
   Dev& d = h->d;
   int coop = 0, smem = 0, sm_smem = 0, reserved = 0;
   if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device) != cudaSuccess || !coop) return 0;
-  if (!sm_count(h)) return 0;
   if (cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device) != cudaSuccess ||
       cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device) != cudaSuccess ||
       cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, h->device) != cudaSuccess)
     return 0;
-  const int G = std::min(std::min(h->sms, kPcgMaxBlocks), h->nslice);
-  const int S = (h->nslice + G - 1) / G;
-  if (S > kPcgMaxSlices) return 0;
   const int words = (h->n + 31) / 32;
-  if ((size_t)words * 8 > 48 * 1024) return 0;
+  if ((size_t)words * 8 + sizeof(int) * kPlanThreads > 48 * 1024) return 0;  // (k_plan_fill's)
   d.pl_ucnt = (int*)dev_alloc(h, sizeof(int) * G);
   d.pl_uown = (int*)dev_alloc(h, sizeof(int) * G);
   if (!d.pl_ucnt || !d.pl_uown) return pcg_no_memory(h);
@@ -1458,13 +1459,16 @@ int run_mixed_dim(lpm_handle* h, bool keep) {
   return 1;
 }
 
+// Most slices of a block in the mixed solve: one to a compute warp.
+int mixed_slices(const lpm_handle* h) { return (h->dim == 3 ? kPcgWideThreads<3> : kPcgWideThreads<2>) / 32 - 1; }
+
 }  // namespace
 
 // The aggregates each block's rows touch (coarse_setup, when the plan is
 // usable): entries (block, aggregate) in two orders, by block and by
 // aggregate, and each row's aggregate among its block's.
 int pcg_coarse_plan(lpm_handle* h, const std::vector<int>& agg, int nagg) {
-  const int st = pcg_plan(h);
+  const int st = pcg_plan(h, mixed_slices(h));
   if (st <= 0) return st < 0 ? st : LPM_OK;
   Dev& d = h->d;
   PcgPlan& pl = h->pcg;
@@ -1511,7 +1515,7 @@ int pcg_coarse_plan(lpm_handle* h, const std::vector<int>& agg, int nagg) {
 }
 
 int pcg_run_mixed(lpm_handle* h, bool keep, bool coarse) {
-  const int st = pcg_plan(h);
+  const int st = pcg_plan(h, mixed_slices(h));
   if (st <= 0) return st;
   if (coarse) return h->dim == 3 ? run_mixed_dim<3, true>(h, keep) : run_mixed_dim<2, true>(h, keep);
   return h->dim == 3 ? run_mixed_dim<3, false>(h, keep) : run_mixed_dim<2, false>(h, keep);

@@ -633,7 +633,6 @@ int run_fp64_dim(lpm_handle* h, const double* A, double* x, double* r, const dou
   Dev& d = h->d;
   PcgPlan& pl = h->pcg;
   using Fn = void (*)(PcgFp64Args);
-  if (pl.S > kPcg64Slices) return 0;
   const Fn fn = keep ? k_pcg_fp64<DIM, true> : k_pcg_fp64<DIM, false>;
   PcgShape& sh = pl.fp64;
   if (!sh.state) sh.state = shape64<DIM>(h, (const void*)fn, &sh) ? 1 : -1;
@@ -678,7 +677,7 @@ int run_fp64_dim(lpm_handle* h, const double* A, double* x, double* r, const dou
 }  // namespace
 
 int pcg_run_fp64(lpm_handle* h, const double* A, double* x, double* r, const double* invd, bool keep) {
-  const int st = pcg_plan(h);
+  const int st = pcg_plan(h, kPcg64Slices);
   if (st <= 0) return st;
   return h->dim == 3 ? run_fp64_dim<3>(h, A, x, r, invd, keep) : run_fp64_dim<2>(h, A, x, r, invd, keep);
 }
