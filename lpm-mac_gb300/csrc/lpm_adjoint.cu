@@ -1235,7 +1235,7 @@ int checkpoint_save(lpm_handle* h, int* id) {
   size_t total = 0;
   for (const CkField& c : f) total += (c.bytes + 255) / 256 * 256;
   void* buf = nullptr;
-  cudaError_t e = cudaMalloc(&buf, std::max<size_t>(total, 256));
+  cudaError_t e = handle_malloc(h, &buf, std::max<size_t>(total, 256));
   if (e != cudaSuccess) {
     cudaGetLastError();
     h->err = "checkpoint: out of device memory";

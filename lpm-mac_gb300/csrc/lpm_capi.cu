@@ -27,9 +27,29 @@ int sm_count(lpm_handle* h) {
   return h->sms;
 }
 
+// The assembly's bond records, which only make it faster, given back for an
+// allocation that did not fit beside them.  (cudaFree waits for the work that
+// reads them.)
+static bool free_records(lpm_handle* h) {
+  if (!h->d.brec) return false;
+  cudaGetLastError();
+  h->allocations.erase(std::find(h->allocations.begin(), h->allocations.end(), (void*)h->d.brec));
+  cudaFree(h->d.brec);
+  h->d.brec = nullptr;
+  h->d.sopp = nullptr;
+  h->no_records = true;
+  return true;
+}
+
+cudaError_t handle_malloc(lpm_handle* h, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && free_records(h)) e = cudaMalloc(p, bytes);
+  return e;
+}
+
 void* dev_alloc(lpm_handle* h, size_t bytes) {
   void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 16));
+  cudaError_t e = handle_malloc(h, &p, std::max<size_t>(bytes, 16));
   if (e != cudaSuccess) {
     cuda_fail(h, e, "cudaMalloc");
     return nullptr;
