@@ -1504,7 +1504,7 @@ int build_mixed_graph(lpm_handle* h, const SellView& sv, const MixedGrids& mg) {
   LPM_CUDA(h, cudaGraphAddNode(&wnode, g, nullptr, nullptr, 0, &wp));
   cudaGraph_t body = wp.conditional.phGraph_out[0];
   const Spmv32Fn spmv = h->mf ? nullptr : spmv32_fn(h, sv);
-  cudaGraphNode_t n_pup;
+  cudaGraphNode_t n_pup = nullptr;
   for (int k = 0; k < kGraphIterations; ++k) {
     const cudaGraphNode_t before = n_pup, *after = k > 0 ? &before : nullptr;
     const bool last = k + 1 == kGraphIterations;
@@ -1577,7 +1577,7 @@ int build_fp64_graph(lpm_handle* h, const double* A, const double* b, double* x,
   wp.conditional.handle = loop_cond;
   wp.conditional.type = cudaGraphCondTypeWhile;
   wp.conditional.size = 1;
-  cudaGraphNode_t wnode, n_spmv, n_upd, n_pup;
+  cudaGraphNode_t wnode, n_spmv, n_upd, n_pup = nullptr;
   LPM_CUDA(h, cudaGraphAddNode(&wnode, g, nullptr, nullptr, 0, &wp));
   cudaGraph_t body = wp.conditional.phGraph_out[0];
   for (int k = 0; k < kGraphIterations; ++k) {
