@@ -736,10 +736,10 @@ struct PcgState {
 // keep the barriers short: a barrier with its fold measured 2.6 us over 152
 // blocks against 4.4 us over 456.
 template <int DIM>
-constexpr int kPcgThreads = DIM == 3 ? 512 : 768;
+constexpr int kMxPersistentThreads = DIM == 3 ? 512 : 768;
 
 template <int DIM, bool OFF16, bool COARSE>
-__global__ void __launch_bounds__(kPcgThreads<DIM>, 1) k_mx_persistent(PcgMixed a) {
+__global__ void __launch_bounds__(kMxPersistentThreads<DIM>, 1) k_mx_persistent(PcgMixed a) {
   __shared__ PcgState s;
   if (threadIdx.x == 0) {
     const CgScalars* c = a.cg;
@@ -1028,10 +1028,10 @@ struct PcgFp64 {
 };
 
 // Most threads per block: the FP64 product's 64 registers, one block per SM.
-constexpr int kPcg64Threads = 1024;
+constexpr int kCgPersistentThreads = 1024;
 
 template <int DIM>
-__global__ void __launch_bounds__(kPcg64Threads, 1) k_cg_persistent(PcgFp64 a) {
+__global__ void __launch_bounds__(kCgPersistentThreads, 1) k_cg_persistent(PcgFp64 a) {
   __shared__ double s_abs_new, s_threshold, s_alpha, s_beta, s_rr;
   __shared__ long long s_it, s_maxit, s_passes;
   __shared__ int s_done;
@@ -1236,7 +1236,7 @@ int run_persistent_fp64(lpm_handle* h, const SellView& sv, const double* A, doub
   using Fn = void (*)(PcgFp64);
   const Fn fn = h->dim == 3 ? k_cg_persistent<3> : k_cg_persistent<2>;
   int threads = 0;
-  const int grid = persistent_shape(h, fn, kPcg64Threads, true, 3, &threads);
+  const int grid = persistent_shape(h, fn, kCgPersistentThreads, true, 3, &threads);
   if (grid <= 0) return 0;
   Dev& d = h->d;
   LPM_CUDA(h, cudaMemsetAsync(d.gbar, 0, sizeof(unsigned long long), h->stream));
@@ -1446,7 +1446,7 @@ int pcg_grid(lpm_handle* h, const SellView& sv, int* threads_out, bool coarse) {
   const bool keep = (long long)h->nslots * h->dim * h->dim * 4 <= kKeepBytes;
   const int mode = h->cg_loop;
   if (coarse) h->cg_loop = LPM_CG_LOOP_PERSISTENT;
-  const int g = persistent_shape(h, pcg_fn(sv, h->dim, coarse), h->dim == 3 ? kPcgThreads<3> : kPcgThreads<2>,
+  const int g = persistent_shape(h, pcg_fn(sv, h->dim, coarse), h->dim == 3 ? kMxPersistentThreads<3> : kMxPersistentThreads<2>,
                                  keep, 7, threads_out);
   h->cg_loop = mode;
   return g;

@@ -475,7 +475,7 @@ __device__ __forceinline__ void coarse_solve(const PcgMixedArgs& a, PcgShared& s
 
 // The e of the block's aggregates, then z of this thread's row (owner).
 template <int DIM>
-__device__ __forceinline__ void coarse_z(const PcgMixedArgs& a, PcgShared& sh, unsigned zn, const Place& pl,
+__device__ __forceinline__ void coarse_row_z(const PcgMixedArgs& a, PcgShared& sh, unsigned zn, const Place& pl,
                                          float (&z)[DIM]) {
   constexpr int NM = kModes<DIM>, E = DIM * DIM;
   const CoarseView<DIM> v = coarse_view<DIM>(a);
@@ -625,7 +625,7 @@ __device__ __noinline__ void reliable_update(const PcgMixedArgs& a) {
   __syncthreads();  // r.z, r.p
   if (COARSE) {
     float z[DIM];
-    coarse_z<DIM>(a, sh, sh.zn + 1, pl, z);
+    coarse_row_z<DIM>(a, sh, sh.zn + 1, pl, z);
     compute_sync(nth);
   }
   if (threadIdx.x == 0) sh.zn += 1;
@@ -1044,7 +1044,7 @@ __device__ __forceinline__ void iterate(const PcgMixedArgs& a) {
     __syncthreads();  // |r|^2, r.z
     if (COARSE) {
       float z[DIM];
-      coarse_z<DIM>(a, sh, zn, pl, z);
+      coarse_row_z<DIM>(a, sh, zn, pl, z);
     }
     // while the sums travel: x += alpha p, and the z of the block's columns
     if (owner) {
@@ -1215,7 +1215,7 @@ __global__ void __launch_bounds__(BOUND, 1) k_pcg_mixed(const __grid_constant__ 
     coarse_solve<DIM>(a, sh, 1, S);
     __syncthreads();
     float z[DIM];
-    coarse_z<DIM>(a, sh, 1, pl, z);
+    coarse_row_z<DIM>(a, sh, 1, pl, z);
     __syncthreads();
     if (st.fail || st.done) return;
   }
