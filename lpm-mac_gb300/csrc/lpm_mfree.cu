@@ -442,9 +442,12 @@ __global__ void __launch_bounds__(256) k_mf_pass1(MfView<T> v, const T* __restri
 // iteration of the mixed solve takes 102 us at 61^3 particles and 343 at 101^3
 // (116 and 348 without; the order alone 108 and 336, the loads alone 103 and
 // 344).  Neither DRAM (2.4 TB/s) nor L2 binds it: the passes wait for the
-// partners' values.
+// partners' values.  In FP64 the sums' registers took a 2-D SM from three blocks
+// to two (86 of them), which cost more than they saved: us per iteration of a
+// 201x401 plate 87 before, 94 then, 83.5 held to three blocks; 401x401 138, 147 and
+// 135; 700x700 319, 336 and 313.
 template <typename T, int DIM, int MODE, bool MASK, int L>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1) k_mf_pass2(MfView<T> v, const T* __restrict__ p, const float* __restrict__ xa,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : DIM == 2 ? 3 : 1) k_mf_pass2(MfView<T> v, const T* __restrict__ p, const float* __restrict__ xa,
                                                   const float* __restrict__ xb, T* __restrict__ q,
                                                   float* __restrict__ qlo, const double* __restrict__ rhs,
                                                   CgScalars* cg, double* partials, unsigned int* ticket) {
