@@ -111,6 +111,16 @@ __device__ __forceinline__ bool grid_fold(const double (&v)[K], double* partials
   return true;
 }
 
+// Sum over the L lanes of a particle, in each of them.  (A particle's lanes
+// are neighbours in a warp and leave a kernel together.)
+template <int L>
+__device__ __forceinline__ double lanes_sum(double v) {
+  const unsigned mask = ((1u << L) - 1u) << ((threadIdx.x & 31) / L * L);
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+  return v;
+}
+
 __device__ __forceinline__ bool is_broken(double bdamage) { return fabs(bdamage - 1.0) < EPS; }
 
 // Particle::distanceTo (particle.h:277-280): sqrt(dx^2 + dy^2 + dz^2) with each

@@ -13,16 +13,6 @@ namespace {
 // Bond geometry + per-layer sums (bond.h:30-39, particle.h:163-181), then
 // the elastic bond force (particle_elastic.h:38-50), which needs the owner's
 // complete dLe_total: bforce = (2 Kn dLe + 2 Tv dLe_total[layer]) (1 - bdamage).
-// Sum over the L lanes of a particle, in each of them.  (A particle's lanes
-// are neighbours in a warp and leave a kernel together.)
-template <int L>
-__device__ __forceinline__ double lanes_sum(double v) {
-  const unsigned mask = ((1u << L) - 1u) << ((threadIdx.x & 31) / L * L);
-#pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
-  return v;
-}
-
 template <int L>
 __global__ void __launch_bounds__(128) k_geometry_force(int n, const double* __restrict__ x, const int64_t* __restrict__ bptr,
                                  const int* __restrict__ bp2, const int* __restrict__ blayer,
@@ -107,16 +97,16 @@ __global__ void __launch_bounds__(128) k_geometry_force(int n, const double* __r
     bforce[b] = f;
     const double c0 = cs[3 * b], c1 = cs[3 * b + 1], c2 = cs[3 * b + 2];
     const double wt = w * Tv[b], wk = w * (2.0 * Kn[b] + Tv[b]);
-    const double t[3] = {wt * c0, wt * c1, wt * c2};
+    const double t[3] = {__dmul_rn(wt, c0), __dmul_rn(wt, c1), __dmul_rn(wt, c2)};
     const double m[6] = {wk * c0 * c0, wk * c0 * c1, wk * c0 * c2, wk * c1 * c1, wk * c1 * c2, wk * c2 * c2};
     if (l1) {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) T[3 + k] += t[k];
+      for (int k = 0; k < 3; ++k) T[3 + k] = __dadd_rn(T[3 + k], t[k]);  // (as k_mf_prep)
 #pragma unroll
       for (int k = 0; k < 6; ++k) M[6 + k] += m[k];
     } else {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) T[k] += t[k];
+      for (int k = 0; k < 3; ++k) T[k] = __dadd_rn(T[k], t[k]);
 #pragma unroll
       for (int k = 0; k < 6; ++k) M[k] += m[k];
     }
@@ -336,21 +326,23 @@ int launch_mean_state0(lpm_handle* h, double* out_dev) {
   return LPM_OK;
 }
 
+// Lanes of a particle.  Where the chip is full the pass is bound by the FP64
+// pipe (some 140 operations a bond, of which the square root and the two
+// quotients are half), and lanes only add their sums; where it is not, by a
+// thread's chain of bonds.  us with 1, 2, 4 and 8 lanes: 1,661 particles of a
+// plate 85, 52, 36, 37; 7,321 87, 54, 50, 78; 28,126 127, 109, 113, 225; cubes
+// of 21^3 120, 67, 69, 87, of 51^3 637, 581, 709, 974, of 101^3 4,165, 4,226,
+// 5,210, 7,379.  So four up to 200 threads on each of the 152 SMs, two up to
+// all they hold.
+int force_lanes(int n) { return n <= 7600 ? 4 : n <= 155000 ? 2 : 1; }
+
 int launch_geometry_force(lpm_handle* h) {
   if (h->tg_ndir > 0 && h->law == LPM_LAW_FATIGUE_HCF) {  // the bond damage's tangent reads it before the pass
     const int st = tangent_hcf_bdamage(h);
     if (st) return st;
   }
   const Dev& d = h->d;
-  // Lanes of a particle.  Where the chip is full the pass is bound by the FP64
-  // pipe (some 140 operations a bond, of which the square root and the two
-  // quotients are half), and lanes only add their sums; where it is not, by a
-  // thread's chain of bonds.  us with 1, 2, 4 and 8 lanes: 1,661 particles of a
-  // plate 85, 52, 36, 37; 7,321 87, 54, 50, 78; 28,126 127, 109, 113, 225; cubes
-  // of 21^3 120, 67, 69, 87, of 51^3 637, 581, 709, 974, of 101^3 4,165, 4,226,
-  // 5,210, 7,379.  So four up to 200 threads on each of the 152 SMs, two up to
-  // all they hold.
-  const int L = h->n <= 7600 ? 4 : h->n <= 155000 ? 2 : 1;
+  const int L = force_lanes(h->n);
   const int T = 128, G = grid_for((long long)h->n * L, T);
   const auto geometry = L == 4 ? k_geometry_force<4> : L == 2 ? k_geometry_force<2> : k_geometry_force<1>;
   const auto particle = L == 4 ? k_particle_force<4> : L == 2 ? k_particle_force<2> : k_particle_force<1>;

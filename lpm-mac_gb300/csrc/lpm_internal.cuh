@@ -301,6 +301,7 @@ namespace lpm {
 
 // ---- kernels launched by the C ABI layer (definitions in the .cu files) ----
 // geometry / force / residual (lpm_force.cu)
+int force_lanes(int n);  // lanes of a warp that share a particle in the force pass: 1, 2 or 4
 int launch_geometry_force(lpm_handle* h);
 int launch_residual(lpm_handle* h, double* norm_r, double* norm_R);
 int launch_move_by_disp(lpm_handle* h);

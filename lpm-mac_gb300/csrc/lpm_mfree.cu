@@ -73,26 +73,30 @@ __global__ void k_mf_slots(int n, const int64_t* __restrict__ bptr, const int* _
 }
 
 // Per assembly: the opposite bond's values in each slot, and S, U, V per
-// particle and layer, in FP64 and FP32.
-__global__ void k_mf_prep(int n, const int64_t* __restrict__ bptr, const int64_t* __restrict__ mbase,
-                          const int* __restrict__ blayer, const int* __restrict__ opp, const double* __restrict__ cs,
-                          const double* __restrict__ bdamage, const double* __restrict__ Kn,
-                          const double* __restrict__ Tv, const double* __restrict__ cs_sum, int64_t ns,
-                          double* __restrict__ m64,
-                          float* __restrict__ m32, double* __restrict__ S64, double* __restrict__ U64,
-                          double* __restrict__ V64, float* __restrict__ S32, float* __restrict__ U32,
-                          float* __restrict__ V32) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// particle and layer, in FP64 and FP32.  U and V add the opposite bonds' n' and
+// t' n' to the sums the force pass made of the bonds' own; for intact bonds the
+// two cancel exactly, since a particle's bonds are shared by the same lanes here
+// (force_lanes) and added in the same order, by the same operations.  (Summing the
+// bonds' own over again here took an assembly of 51^3 particles from 480 to 600 us,
+// of 70^3 from 1.15 to 1.66 ms; so it is 458 us and 1.11 ms.)
+template <int L>
+__global__ void __launch_bounds__(128) k_mf_prep(int n, const int64_t* __restrict__ bptr,
+                                                 const int64_t* __restrict__ mbase, const int* __restrict__ blayer,
+                                                 const int* __restrict__ opp, const double* __restrict__ cs,
+                                                 const double* __restrict__ bdamage, const double* __restrict__ Kn,
+                                                 const double* __restrict__ Tv, const double* __restrict__ cs_sum,
+                                                 const double* __restrict__ tsum, int64_t ns, double* __restrict__ m64,
+                                                 float* __restrict__ m32, double* __restrict__ S64,
+                                                 double* __restrict__ U64, double* __restrict__ V64,
+                                                 float* __restrict__ S32, float* __restrict__ U32,
+                                                 float* __restrict__ V32) {
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L), sub = threadIdx.x % L;
   if (i >= n) return;
   const int64_t s0 = mbase[i / 32] + (i % 32);
-  // sums of the opposite bonds' n' and t' n', and of the bonds' own in the same
-  // order: for intact bonds the two cancel exactly
   double so[NL][3] = {{0, 0, 0}, {0, 0, 0}}, to[NL][3] = {{0, 0, 0}, {0, 0, 0}};
-  double sn[NL][3] = {{0, 0, 0}, {0, 0, 0}}, tn[NL][3] = {{0, 0, 0}, {0, 0, 0}};
-  int k = 0;
-  for (int64_t b = bptr[i]; b < bptr[i + 1]; ++b, ++k) {
+  int k = sub;
+  for (int64_t b = bptr[i] + sub; b < bptr[i + 1]; b += L, k += L) {
     const int bo = opp[b];
-    const double to1 = (1.0 - bdamage[b]) * Tv[b];
     const double w = 1.0 - bdamage[bo], tv = Tv[bo];
     const double tp = w * tv, c1 = w * (2.0 * Kn[bo] + tv) - tp;
     const double v[kMfFields] = {cs[3 * (int64_t)bo], cs[3 * (int64_t)bo + 1], cs[3 * (int64_t)bo + 2], c1, tp};
@@ -102,13 +106,15 @@ __global__ void k_mf_prep(int n, const int64_t* __restrict__ bptr, const int64_t
     // FP32: one 16-byte word {n'x, n'y, n'z, t'} per slot, then a' - t'
     reinterpret_cast<float4*>(m32)[slot] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)tp);
     m32[4 * ns + slot] = (float)c1;
-    const int l = blayer[b] != 0;
+    const bool l1 = blayer[b] != 0;  // (the layer's sums by selection: in registers)
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      so[l][c] += v[c];
-      to[l][c] += tp * v[c];
-      sn[l][c] += cs[3 * b + c];
-      tn[l][c] += to1 * cs[3 * b + c];
+      const double s = (l1 ? so[1][c] : so[0][c]) + v[c];
+      const double t = __dadd_rn(l1 ? to[1][c] : to[0][c], __dmul_rn(tp, v[c]));
+      so[0][c] = l1 ? so[0][c] : s;
+      so[1][c] = l1 ? s : so[1][c];
+      to[0][c] = l1 ? to[0][c] : t;
+      to[1][c] = l1 ? t : to[1][c];
     }
   }
 #pragma unroll
@@ -116,7 +122,8 @@ __global__ void k_mf_prep(int n, const int64_t* __restrict__ bptr, const int64_t
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int64_t q = ((int64_t)i * NL + l) * 3 + c;
-      const double S = cs_sum[q], U = sn[l][c] + so[l][c], V = tn[l][c] + to[l][c];
+      const double S = cs_sum[q], U = S + lanes_sum<L>(so[l][c]), V = tsum[q] + lanes_sum<L>(to[l][c]);
+      if (sub) continue;
       S64[q] = S;
       U64[q] = U;
       V64[q] = V;
@@ -781,9 +788,11 @@ int mf_assemble(lpm_handle* h, int tangent, int bc) {
     if (st) return st;
   }
   const int n = h->n;
-  k_mf_prep<<<grid_for(n, 128), 128, 0, h->stream>>>(n, d.bptr, d.mbase, d.blayer, d.opp, d.cs, d.bdamage, d.Kn,
-                                                      d.Tv, d.cs_sum, h->mslots, d.m64, d.m32, d.mS64, d.mU64,
-                                                      d.mV64, d.mS32, d.mU32, d.mV32);
+  const int L = force_lanes(n);
+  const auto prep = L == 4 ? k_mf_prep<4> : L == 2 ? k_mf_prep<2> : k_mf_prep<1>;
+  prep<<<grid_for((long long)n * L, 128), 128, 0, h->stream>>>(n, d.bptr, d.mbase, d.blayer, d.opp, d.cs, d.bdamage,
+                                                               d.Kn, d.Tv, d.cs_sum, d.tsum, h->mslots, d.m64, d.m32,
+                                                               d.mS64, d.mU64, d.mV64, d.mS32, d.mU32, d.mV32);
   LPM_LAUNCHED(h, "k_mf_prep");
   k_mf_flags<<<grid_for(n, 128), 128, 0, h->stream>>>(n, d.mbase, d.mU64, d.mV64, d.mp2);
   LPM_LAUNCHED(h, "k_mf_flags");
