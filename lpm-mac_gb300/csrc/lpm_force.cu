@@ -3,8 +3,9 @@
 //
 // One, two or four lanes of a warp own a particle (launch_geometry_force) and
 // take its bonds in stored order in turn (Particle::bond_layers,
-// particle.h:163-181, 197-240); a bond's own values are the same with any
-// number of lanes, a particle's sums are the lanes' added in a fixed order.
+// particle.h:163-181, 197-240); a bond's length, strain, stretch and direction
+// are the same with any number of lanes, a particle's sums are the lanes' added
+// in a fixed order, and the bond force, which has a layer's sum in it, follows them.
 #include "lpm_device.cuh"
 
 namespace lpm {
