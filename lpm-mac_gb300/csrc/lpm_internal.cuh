@@ -200,7 +200,7 @@ struct Dev {
   double *tg_dD, *tg_ddot, *tg_dnl;
   // on-chip CG solves (lpm_pcg.cu): per block the columns its rows need,
   // their count and the position of its first row among them, per slot the
-  // column's position; (z, p) of every row, twice; the barriers' words
+  // column's position; z of every row in records, twice; the records of the sums
   int *pl_ucnt, *pl_uown, *pl_ulist;
   unsigned short* pl_lidx;
   float* pl_zp;

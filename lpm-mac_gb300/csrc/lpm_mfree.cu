@@ -474,11 +474,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : DIM == 2 ? 3 : 1) k_
       for (int r = 0; r < DIM; ++r)
 #pragma unroll
         for (int c = 0; c < DIM; ++c) {
-        if constexpr (sizeof(T) == 4)
-          dot2_acc(ys[r], yc[r], Ri[r * 3 + c], pi[c]);
-        else
-          ys[r] = fma(Ri[r * 3 + c], pi[c], ys[r]);
-      }
+          if constexpr (sizeof(T) == 4)
+            dot2_acc(ys[r], yc[r], Ri[r * 3 + c], pi[c]);
+          else
+            ys[r] = fma(Ri[r * 3 + c], pi[c], ys[r]);
+        }
     const int sl = i / 32;
     const int64_t s0 = v.mbase[sl] + (i % 32) + 32 * part;
     const int len = ((int)((v.mbase[sl + 1] - v.mbase[sl]) / 32) - part + L - 1) / L;  // this lane's slots
@@ -704,7 +704,11 @@ MfView<T> mf_view(lpm_handle* h) {
 // only adds its sums, and in FP64 the passes are bound by its pipe earlier.  us
 // per iteration with one, two and four lanes: mixed solve, 21^3 particles 43.5,
 // 36.8, 33.6; 41^3 55, 47, 53; 61^3 90, 88, 103; 101^3 287, 308, 372; FP64 solve,
-// 21^3 64, 45, 37; 41^3 109, 116, 139; 61^3 288, 306, 378.
+// 21^3 64, 45, 37; 41^3 109, 116, 139; 61^3 288, 306, 378.  Plates, with one and two:
+// mixed solve, 1,661 particles 28.8 and 25.9, 34k 33.2 and 28.7, 80k 38.9 and 38.8,
+// 230k 60.8 and 61.1, 308k 65.5 and 77.0; FP64 solve 37.9 and 28.7, 41.0 and 42.5,
+// 95.4 and 86.7 (with two blocks an SM), 168 and 187.  So two lanes up to what the
+// 152 SMs hold of threads, once over (FP64: a tenth of that).
 int mf_lanes(const lpm_handle* h, bool fp32) { return h->n <= (fp32 ? 311000 : 32000) ? 2 : 1; }
 
 // Grid of the two passes: grid-stride, at most as many blocks as the

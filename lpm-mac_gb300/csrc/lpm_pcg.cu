@@ -14,8 +14,9 @@
 //     their halo, at most a few thousand) is staged into shared memory once
 //     per iteration, so that a block's value is fetched by its 16-bit
 //     position there;
-//   - the row's vectors (r, x, z and p, the first two as double-float pairs)
-//     stay in the registers of the warp that owns its slice;
+//   - the row's residual, a double-float pair, and its product stay in the
+//     registers of the warp that owns its slice (x, a pair too, is updated in
+//     global memory while the sums travel);
 //   - two grid barriers per iteration instead of three: the new direction
 //     p = zc z + beta p is formed by every block from the z and the old p of
 //     the columns it stages, not written by the owner and read back;
@@ -1433,7 +1434,6 @@ int run_mixed_dim(lpm_handle* h, bool keep) {
   a.off_row = sh.off_row;
   a.off_coarse = sh.off_coarse;
   a.off_op = sh.off_op;
-  // tags start at 1
   if (COARSE) {
     a.nc = h->cnc;
     a.cmaxrows = cmaxrows;
@@ -1451,6 +1451,7 @@ int run_mixed_dim(lpm_handle* h, bool keep) {
     LPM_CUDA(h, cudaMemsetAsync(d.pc_rec, 0, 16 * 2 * ((size_t)pl.centries * kModes<DIM> + 2 * (size_t)h->cnc),
                                 h->stream));
   }
+  // the records' tags, which start at 1
   LPM_CUDA(h, cudaMemsetAsync(d.pl_words, 0, kWordBytes, h->stream));
   LPM_CUDA(h, cudaMemsetAsync(d.pl_zp, 0, kZBytes * (size_t)h->n, h->stream));
   void* args[] = {&a};

@@ -9,7 +9,8 @@ namespace lpm {
 constexpr int kPcgMaxBlocks = 160;  // blocks of a solve, at most one per SM (GB300: 152)
 constexpr int kPcgMaxSlices = 32;   // 32-row slices of a block (a lane each in its sums)
 
-// Threads per block, one block per SM, the message warp included: registers
+// Most threads per block, the message warp included (of an SM to itself; small
+// systems take less, shape_on_plan): registers
 // for an operator group in flight beside the one in use (2-D: 80, 3-D: 128).
 // The wide form has a warp more for 2-D blocks of 24 slices (72 registers),
 // the narrow one 128 registers in 2-D too: at 80 the message warp keeps part of

@@ -665,7 +665,7 @@ int run_fp64_dim(lpm_handle* h, const double* A, double* x, double* r, const dou
   a.off_row = sh.off_row;
   a.off_tail = sh.off_coarse;
   a.off_op = sh.off_op;
-  // tags start at 1
+  // the records' tags, which start at 1
   LPM_CUDA(h, cudaMemsetAsync(d.pl_words, 0, kWordBytes, h->stream));
   LPM_CUDA(h, cudaMemsetAsync(d.pl_zp, 0, kZBytes64 * (size_t)h->n, h->stream));
   void* args[] = {&a};

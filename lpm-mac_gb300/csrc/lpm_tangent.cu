@@ -334,6 +334,19 @@ __device__ __forceinline__ void off_block(const AsmView& v, int i, int j, double
   }
 }
 
+template <int DIM, bool REC>
+__device__ __forceinline__ void store_block(const AsmView& v, int64_t slot, int i, int j) {
+  double K[3][3];
+  if (i == j)
+    diag_block<DIM>(v, i, K);
+  else
+    off_block<DIM, REC>(v, i, j, K);
+#pragma unroll
+  for (int r = 0; r < DIM; ++r)
+#pragma unroll
+    for (int s = 0; s < DIM; ++s) v.A[(r * DIM + s) * v.nslots + slot] = K[s][r];
+}
+
 // A block per slice of A = K^T: lane t owns row j = 32*slice + t, the warps
 // share the row's blocks.  Each block K_ij is computed by its row's lane and
 // its transpose stored in the row's slot.
@@ -354,18 +367,6 @@ __device__ __forceinline__ void off_block(const AsmView& v, int i, int j, double
 // the raw arrays, then with the warps and the records, then by offsets: a 7k
 // plate 333, 82 and 67 us, a 21^3 cube 1203, 258 and 180 us, 51^3 2914, 1559
 // and 1080 us, 101^3 17.8, 8.9 and 7.3 ms.
-template <int DIM, bool REC>
-__device__ __forceinline__ void store_block(const AsmView& v, int64_t slot, int i, int j) {
-  double K[3][3];
-  if (i == j)
-    diag_block<DIM>(v, i, K);
-  else
-    off_block<DIM, REC>(v, i, j, K);
-#pragma unroll
-  for (int r = 0; r < DIM; ++r)
-#pragma unroll
-    for (int s = 0; s < DIM; ++s) v.A[(r * DIM + s) * v.nslots + slot] = K[s][r];
-}
 template <int DIM, bool REC>
 __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmView v, int noff) {
   extern __shared__ int off[];  // [noff], ascending
