@@ -700,16 +700,16 @@ MfView<T> mf_view(lpm_handle* h) {
 
 // Lanes of a particle in the passes.  With one, 61^3 particles are 1.5 waves of
 // resident threads, and a thread's chain of slots sets the time; with two the
-// waves are shorter and more even.  Where there are many waves the second lane
-// only adds its sums, and in FP64 the passes are bound by its pipe earlier.  us
-// per iteration with one, two and four lanes: mixed solve, 21^3 particles 43.5,
-// 36.8, 33.6; 41^3 55, 47, 53; 61^3 90, 88, 103; 101^3 287, 308, 372; FP64 solve,
-// 21^3 64, 45, 37; 41^3 109, 116, 139; 61^3 288, 306, 378.  Plates, with one and two:
-// mixed solve, 1,661 particles 28.8 and 25.9, 34k 33.2 and 28.7, 80k 38.9 and 38.8,
-// 230k 60.8 and 61.1, 308k 65.5 and 77.0; FP64 solve 37.9 and 28.7, 41.0 and 42.5,
-// 95.4 and 86.7 (with two blocks an SM), 168 and 187.  So two lanes up to what the
-// 152 SMs hold of threads, once over (FP64: a tenth of that).
-int mf_lanes(const lpm_handle* h, bool fp32) { return h->n <= (fp32 ? 311000 : 32000) ? 2 : 1; }
+// waves are shorter and more even.  Past that the second lane only adds its sums
+// (and past 262,144 particles the grid's 2,048 blocks take a second turn), and in
+// FP64 the passes are bound by its pipe earlier.  us per iteration with one and
+// two lanes: mixed solve, cubes of 21^3 particles 43.5 and 36.8, 31^3 45 and 35, 58^3
+// 76 and 74, 61^3 84 and 82, 63^3 87 and 90, 65^3 89 and 100, 101^3 287 and 308;
+// plates of 1,661 particles 28.8 and 25.9, 34k 33.2 and 28.7, 80k 37.6 and 37.6, 202k
+// 59 and 58, 230k 61 and 61, 260k 63 and 68; FP64 solve, 21^3 64 and 45, 31^3 62 and
+// 63, 63^3 319 and 326, plates of 1,661 38 and 29, 30k 40 and 41, 80k 84 and 81, 260k
+// 185 and 202.  Four lanes: 21^3 33.6 and 37, but 41^3 53 and 139 against 47 and 109.
+int mf_lanes(const lpm_handle* h, bool fp32) { return h->n <= (fp32 ? 240000 : 32000) ? 2 : 1; }
 
 // Grid of the two passes: grid-stride, at most as many blocks as the
 // reduction partials hold.
