@@ -27,14 +27,20 @@ int sm_count(lpm_handle* h) {
   return h->sms;
 }
 
+void dev_free(lpm_handle* h, void* p) {
+  auto& a = h->allocations;
+  a.erase(std::remove(a.begin(), a.end(), p), a.end());
+  cudaFree(p);
+}
+
 // The assembly's bond records, which only make it faster, given back for an
 // allocation that did not fit beside them.  (cudaFree waits for the work that
 // reads them.)
 static bool free_records(lpm_handle* h) {
   if (!h->d.brec) return false;
   cudaGetLastError();
-  h->allocations.erase(std::find(h->allocations.begin(), h->allocations.end(), (void*)h->d.brec));
-  cudaFree(h->d.brec);
+  dev_free(h, h->d.brec);
+  dev_free(h, h->d.sopp);
   h->d.brec = nullptr;
   h->d.sopp = nullptr;
   h->no_records = true;

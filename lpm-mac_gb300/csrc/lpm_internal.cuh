@@ -379,6 +379,7 @@ void set_global_error(const std::string& msg);  // text of lpm_last_error(NULL)
 int sm_count(lpm_handle* h);  // multiprocessors of the handle's device, looked up once; 0 if that fails
 cudaError_t handle_malloc(lpm_handle* h, void** p, size_t bytes);  // cudaMalloc; gives up what the handle can do without
 void* dev_alloc(lpm_handle* h, size_t bytes);
+void dev_free(lpm_handle* h, void* p);  // an allocation of dev_alloc, before the handle's end
 void* zeros_dev(lpm_handle* h, size_t bytes);  // dev_alloc + zero fill
 // Blocks for `work` threads.  No cap unless the kernel loops with a grid stride:
 // one that does not would leave out what lies past it.

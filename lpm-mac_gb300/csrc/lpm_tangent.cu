@@ -636,17 +636,20 @@ static int bond_records(lpm_handle* h) {
   if (h->no_records || h->nb == 0) return 0;
   const int T = 256, G = grid_for((long long)h->nb, T, 152 * 32);
   if (!d.brec) {
-    // the records, then each one's opposite; given back where memory runs short
-    // later (handle_malloc)
-    d.brec = (double*)dev_alloc(h, (sizeof(double) * 4 + sizeof(int)) * (size_t)h->nb);
-    int* place = nullptr;
-    if (!d.brec || cudaMallocAsync((void**)&place, sizeof(int) * (size_t)h->nb, h->stream) != cudaSuccess) {
+    // the records and each one's opposite; given back where memory runs short later
+    // (handle_malloc)
+    double* rec = (double*)dev_alloc(h, sizeof(double) * 4 * (size_t)h->nb);
+    int *sopp = rec ? (int*)dev_alloc(h, sizeof(int) * (size_t)h->nb) : nullptr, *place = nullptr;
+    if (!sopp || cudaMallocAsync((void**)&place, sizeof(int) * (size_t)h->nb, h->stream) != cudaSuccess) {
       cudaGetLastError();
       h->err.clear();
       h->no_records = true;
+      if (sopp) dev_free(h, sopp);
+      if (rec) dev_free(h, rec);
       return 0;
     }
-    d.sopp = (int*)(d.brec + 4 * (size_t)h->nb);
+    d.brec = rec;
+    d.sopp = sopp;
     k_sorted_place<<<G, T, 0, h->stream>>>(h->nb, d.sbond, place);
     LPM_LAUNCHED(h, "k_sorted_place");
     k_sorted_opp<<<G, T, 0, h->stream>>>(h->nb, d.sbond, d.opp, place, d.sopp);
