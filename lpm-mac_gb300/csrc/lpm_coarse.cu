@@ -155,21 +155,28 @@ __global__ void __launch_bounds__(kPairThreads) k_coarse_pairs(const int* __rest
 // First, modes without stiffness (a diagonal entry at most 1e-12 of the
 // largest) are set aside: their rows and columns become the identity's for
 // the elimination, and the inverse's are cleared; `active` records which
-// are kept.  The result is symmetrized, (B + B^T)/2, into the other buffer
+// are kept.  A mode that the ones before it span (an aggregate with fewer free
+// DOFs than modes) shows as a pivot of nothing but rounding, 1e-16 of the mode's
+// diagonal entry, where those of slender bars still have 4e-6: at most kDependent
+// of it, the mode is set aside then.  (P A_c^-1 P^T is that of the modes' space,
+// whichever of them span it.)  The result is symmetrized, (B + B^T)/2, into the other buffer
 // (X after an odd number of steps, else Y): elimination leaves the computed
 // inverse of an ill-conditioned A_c slightly unsymmetric, and CG needs a
 // symmetric preconditioner.
 constexpr int kInv = 16;         // columns per step
 constexpr int kInvRows = 16, kInvCols = 32;  // tile of the update
 constexpr int kInvThreads = 256;
+constexpr double kDependent = 1e-13;
 
 // D^-1 of the block of step k after the update of step k - 1 (k > 0) applied
-// to it, into dinv (global, kInv x kInv, identity beyond the matrix).
+// to it, into dinv (global, kInv x kInv, identity beyond the matrix and for modes
+// set aside; diag: the modes' diagonal entries).
 __device__ void invert_diagonal(int nc, int k, const double* src, const double* panel, double* dinv,
-                                double (&d)[kInv][kInv + 1]) {
+                                double (&d)[kInv][kInv + 1], const double* diag, int* active) {
   const int r = threadIdx.x / kInv, c = threadIdx.x % kInv, i = k * kInv + r, j = k * kInv + c;
   const bool in = i < nc && j < nc;
   __shared__ double rp;
+  __shared__ int dependent;
   double v = in ? __ldcg(&src[(int64_t)i * nc + j]) : (r == c ? 1.0 : 0.0);
   if (panel && in) {  // A_ij - A_i(k-1) P
     const int k0 = (k - 1) * kInv;
@@ -179,11 +186,19 @@ __device__ void invert_diagonal(int nc, int k, const double* src, const double* 
   d[r][c] = v;
   __syncthreads();
   for (int p = 0; p < kInv; ++p) {
-    if (threadIdx.x == 0) rp = 1.0 / d[p][p];
+    if (threadIdx.x == 0) {
+      const int m = k * kInv + p;
+      dependent = m < nc && fabs(d[p][p]) <= kDependent * fabs(__ldcg(&diag[m]));
+      if (dependent) active[m] = 0;
+      rp = 1.0 / d[p][p];
+    }
     __syncthreads();
     const double q = rp, a = d[r][c], f = d[r][p], g = d[p][c];
+    const bool aside = dependent;
     __syncthreads();
-    if (r == p)
+    if (aside)
+      d[r][c] = r != p && c != p ? a : r == c ? 1.0 : 0.0;
+    else if (r == p)
       d[r][c] = c == p ? q : a * q;
     else
       d[r][c] = c == p ? -a * q : a - f * q * g;
@@ -193,7 +208,7 @@ __device__ void invert_diagonal(int nc, int k, const double* src, const double* 
 }
 
 __global__ void __launch_bounds__(kInvThreads) k_coarse_invert(int nc, double* X, double* Y, double* dinv,
-                                                               int* __restrict__ active, unsigned long long* gbar,
+                                                               double* diag, int* active, unsigned long long* gbar,
                                                                long long spin_limit, int* fault) {
   __shared__ double D[kInv][kInv + 1], L[kInvRows][kInv + 1], P[kInv][kInvCols];
   __shared__ double smax[kInvThreads / 32];
@@ -217,7 +232,11 @@ __global__ void __launch_bounds__(kInvThreads) k_coarse_invert(int nc, double* X
     __syncthreads();
     m = 0.0;
     for (int w = 0; w < kInvThreads / 32; ++w) m = fmax(m, smax[w]);
-    for (int64_t q = t0; q < nc; q += stride) active[q] = fabs(__ldcg(&X[q * nc + q])) > 1e-12 * m ? 1 : 0;
+    for (int64_t q = t0; q < nc; q += stride) {
+      const double a = __ldcg(&X[q * nc + q]);
+      active[q] = fabs(a) > 1e-12 * m ? 1 : 0;
+      diag[q] = active[q] ? a : 1.0;
+    }
     if (!barrier()) return;
     for (int64_t e = t0; e < nn; e += stride) {
       const int r = (int)(e / nc), c = (int)(e % nc);
@@ -225,7 +244,7 @@ __global__ void __launch_bounds__(kInvThreads) k_coarse_invert(int nc, double* X
     }
     if (!barrier()) return;
   }
-  if (blockIdx.x == last) invert_diagonal(nc, 0, X, nullptr, dinv, D);
+  if (blockIdx.x == last) invert_diagonal(nc, 0, X, nullptr, dinv, D, diag, active);
   if (!barrier()) return;
   const int steps = (nc + kInv - 1) / kInv;
   const int rows = (nc + kInvRows - 1) / kInvRows, cols = (nc + kInvCols - 1) / kInvCols;
@@ -241,21 +260,22 @@ __global__ void __launch_bounds__(kInvThreads) k_coarse_invert(int nc, double* X
       double v = 0.0;
       if (j >= k0 && j < k0 + kb) {
         v = __ldcg(&dk[r * kInv + j - k0]);
-      } else {
+      } else if (__ldcg(&active[k0 + r])) {
         for (int t = 0; t < kb; ++t) v += __ldcg(&dk[r * kInv + t]) * __ldcg(&src[(int64_t)(k0 + t) * nc + j]);
       }
       dst[(int64_t)(k0 + r) * nc + j] = v;
     }
     if (!barrier()) return;
     if ((int)blockIdx.x == last && k + 1 < steps)
-      invert_diagonal(nc, k + 1, src, dst, dinv + ((k + 1) & 1) * kInv * kInv, D);
+      invert_diagonal(nc, k + 1, src, dst, dinv + ((k + 1) & 1) * kInv * kInv, D, diag, active);
     if ((int)blockIdx.x < workers)
       for (int tile = blockIdx.x; tile < rows * cols; tile += workers) {
         const int i0 = tile / cols * kInvRows, j0 = tile % cols * kInvCols;
         __syncthreads();
         for (int e = threadIdx.x; e < kInvRows * kInv; e += kInvThreads) {
           const int r = e / kInv, t = e % kInv;
-          L[r][t] = i0 + r < nc && t < kb ? __ldcg(&src[(int64_t)(i0 + r) * nc + k0 + t]) : 0.0;
+          L[r][t] = i0 + r < nc && t < kb && __ldcg(&active[k0 + t]) ? __ldcg(&src[(int64_t)(i0 + r) * nc + k0 + t])
+                                                                      : 0.0;
         }
         // the k-th columns take D^-1 (in dst's row panel) and start from zero
         for (int e = threadIdx.x; e < kInv * kInvCols; e += kInvThreads) {
@@ -278,7 +298,7 @@ __global__ void __launch_bounds__(kInvThreads) k_coarse_invert(int nc, double* X
   double* out = (steps & 1) ? X : Y;
   for (int64_t e = t0; e < nn; e += stride) {
     const int i = (int)(e / nc), j = (int)(e % nc);
-    out[e] = (!active[i] || !active[j]) ? 0.0 : 0.5 * (__ldcg(&res[e]) + __ldcg(&res[(int64_t)j * nc + i]));
+    out[e] = (!__ldcg(&active[i]) || !__ldcg(&active[j])) ? 0.0 : 0.5 * (__ldcg(&res[e]) + __ldcg(&res[(int64_t)j * nc + i]));
   }
 }
 
@@ -520,7 +540,8 @@ int coarse_assemble(lpm_handle* h) {
   LPM_CUDA(h, cudaMemsetAsync(d.cfault, 0, sizeof(int), h->stream));
   long long spin = kPcgSpinLimit;
   int ncv = nc;
-  void* args[] = {&ncv, &d.cA, &d.cA2, &d.cdinv, &d.cact, &d.gbar, &spin, &d.cfault};
+  // (d.cyc, the solves' y, holds the diagonal meanwhile)
+  void* args[] = {&ncv, &d.cA, &d.cA2, &d.cdinv, &d.cyc, &d.cact, &d.gbar, &spin, &d.cfault};
   LPM_CUDA(h, cudaLaunchCooperativeKernel((const void*)k_coarse_invert, dim3(grid), dim3(kInvThreads), args, 0,
                                           h->stream));
   LPM_LAUNCHED(h, "k_coarse_invert");
