@@ -83,7 +83,9 @@ def test_edge_cases_run_on_chip(precision):
 
 
 # size: slices of the largest of 152 blocks
-ON_CHIP_FP64 = {"plate 120x120": (2, (120, 120), 0),    # 3
+ON_CHIP_FP64 = {"plate 61x121": (2, (61, 121), 0),      # 2, seven warps, two blocks an SM
+                "plate 91x105": (2, (91, 105), 0),      # 2
+                "plate 120x120": (2, (120, 120), 0),    # 3
                 "plate 140x170": (2, (140, 170), 0),    # 5
                 "plate 190x190": (2, (190, 190), 0),    # 8, eight warps
                 "plate 190x210": (2, (190, 210), 0),    # 9, twelve
@@ -92,7 +94,9 @@ ON_CHIP_FP64 = {"plate 120x120": (2, (120, 120), 0),    # 3
                 "box 24x25x26": (3, (24, 25, 26), 0),   # 4
                 "box 30x30x30": (3, (30, 30, 30), 0),   # 6
                 "box 38x38x38": (3, (38, 38, 38), 0)}   # 12
-ON_CHIP_MIXED = {"box 35x35x35": (3, (35, 35, 35), 0),  # 9
+ON_CHIP_MIXED = {"plate 61x121": (2, (61, 121), 0),     # 2, six warps, two blocks an SM
+                 "box 12x13x14": (3, (12, 13, 14), 0),  # 1, seven
+                 "box 35x35x35": (3, (35, 35, 35), 0),  # 9
                  "box 38x38x38": (3, (38, 38, 38), 0),  # 12
                  "box 41x41x41": (3, (41, 41, 41), 0)}  # 15
 
