@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(kPcg64Threads, 1) k_pcg_fp64(const __grid_cons
 // here against there: 44k rows, ten slices, 34.1 (31.7), 45.9k 34.4 (31.6), 50.3k,
 // eleven, 37.8 (32.8), 52k 38.0 (32.3); within windows of 16,384 particles (24 to 27
 // columns) the two are even, 45.9k 31.7 (31.6), or this is ahead, 57.8k 31.9
-// (34.8).  Up to nine slices it depends on the box: 23.7k rows 23.0 (24.5), 33.9k
+// (34.8).  Up to nine slices either may be ahead: 23.7k rows 23.0 (24.5), 33.9k
 // 28.8 (29.1 to 29.7), 39.8k 29.3 or 32.1 (30.7).  In 3-D, nine elements to a block,
 // what fits is ahead: 26^3 at random, 47 columns a row, 37.4 (69.4).
 constexpr int kColumnsPerRow = 26, kColumnsSlices = 9;
